@@ -214,3 +214,54 @@ def tolerance(case):
     attention paths show 0.0023 to 0.0034 and 0.012 to 0.026 (Q and K rounded to bf16 after the norm and the
     rotation, P and O rounded to bf16), the row kernels 0.0020 and 0.013 (two roundings)."""
     return {"rel": 8e-3, "max": 5e-2} if case["path"] == "rows" else {"rel": 1.2e-2, "max": 8e-2}
+
+
+def _turned(x, gain, cos, sin):
+    """RMSNorm over each head row times the gain, then the rotation of interleaved pairs, in 64 bits."""
+    x = x.cuda().double()
+    x = x * torch.rsqrt((x * x).mean(-1, keepdim=True) + RMS_EPS) * gain.double()
+    even, odd = x[..., 0::2], x[..., 1::2]
+    c, s = cos.double()[:, None, :], sin.double()[:, None, :]
+    return torch.stack([even * c - odd * s, even * s + odd * c], dim=-1).flatten(-2)
+
+
+def _attended(q, k, v):
+    """softmax(Q K^T / sqrt(128)) V of [batch, tokens, heads, 128], in 64 bits, a block of rows of one head at a time."""
+    out = torch.empty_like(q)
+    for b in range(q.shape[0]):
+        for h in range(q.shape[2]):
+            keys, values = k[b, :, h].T.contiguous(), v[b, :, h].cuda().double()
+            for r in range(0, q.shape[1], 4096):
+                scores = (q[b, r:r + 4096, h] @ keys).mul_(D ** -0.5)
+                out[b, r:r + 4096, h] = torch.softmax(scores, -1) @ values
+    return out
+
+
+def exact(case, seed):
+    """The outputs of run() for these inputs in 64 bits, without the bf16 roundings between the steps."""
+    s = prepare(case, seed)
+    St = case["txt"]
+
+    def joint(a, gains, tables):
+        q = torch.cat([_turned(a[0], gains[0], *tables[:2]), _turned(a[3], gains[2], *tables[2:])], 1)
+        k = torch.cat([_turned(a[1], gains[1], *tables[:2]), _turned(a[4], gains[3], *tables[2:])], 1)
+        o = _attended(q, k, torch.cat([a[2], a[5]], 1))
+        return [o[:, :St], o[:, St:]]
+
+    if case["path"] in ("joint", "host"):
+        return joint(s["args"], s["gains"], s["tables"])
+    if case["path"] == "single":
+        q, k, v = s["args"]
+        return _attended(_turned(q, s["gains"][0], *s["tables"]), _turned(k, s["gains"][1], *s["tables"]), v)
+    if case["path"] == "plain":
+        q, k, v = s["args"]
+        return _attended(q.double(), k.double(), v)
+    if case["path"] == "step":
+        doubles, singles, gains, tables, combined = s["keep"]
+        outs = []
+        for c in doubles:
+            outs += joint((c.q_txt, c.k_txt, c.v_txt, c.q_img, c.k_img, c.v_img), gains, tables)
+        for c in singles:
+            outs.append(_attended(_turned(c.q, gains[2], *combined), _turned(c.k, gains[3], *combined), c.v))
+        return outs
+    return _turned(s["x"], s["gain"], s["cos"], s["sin"])
