@@ -4,31 +4,41 @@
 // key/value tile of the attended sequence. Three warpgroups:
 //
 //   warps 0-3 / 4-7     softmax group for tile 0 / tile 1: one thread per query
-//                       row (= TMEM lane). Reads S_t with tcgen05.ld, keeps the
-//                       row in registers, exponentiates in the log2 domain, writes
-//                       bf16 P_t over the first 64 columns of S_t (handed to the MMA
-//                       warp in parts, so P_t V_j starts before the row is finished)
-//                       and accumulates the row sum from the unrounded fp32 values.
+//                       row (= TMEM lane). Reads S with tcgen05.ld, keeps the row in
+//                       registers, exponentiates in the log2 domain, writes bf16 P_t to
+//                       its 64 columns (handed to the MMA warp in halves, so P_t V_j
+//                       starts before the row is finished) and accumulates the row sum
+//                       from the unrounded fp32 values.
 //   warp 8  (one lane)  TMA producer: Q tiles once, then K_j, V_j into a 4-slot
 //                       ring of 32 KiB shared-memory slots (mbarrier full/empty).
-//   warp 9  (converged) tcgen05.mma issuer:  S_t = Q_t K_j^T  (A, B from shared
+//   warp 9  (converged) tcgen05.mma issuer:  S = Q_t K_j^T  (A, B from shared
 //                       memory, K-major, 128-byte swizzle) and O_t += P_t V_j
-//                       (A = P_t from tensor memory, B = V_j MN-major). S_0, S_1,
-//                       O_0, O_1 are 128-column fp32 accumulators in TMEM.
+//                       (A = P_t from tensor memory, B = V_j MN-major).
 //   warps 10-11         give their registers to the softmax groups (setmaxnreg: 208 registers
 //                       per softmax thread, 88 elsewhere). In head-exchange use they do the
 //                       exchange: QK-norm + RoPE of this rank's raw Q, K and peer stores of every
 //                       head row to the rank that attends it, while the other roles already work
 //                       on what has arrived (ExchangeParams). Idle otherwise.
 //
-// Issue order per key/value tile j:  S0_j, PV1_{j-1}, S1_j, PV0_j.  While one
-// softmax group works on its S, the tensor pipe runs the other tile's two MMAs.
+// Tensor memory (512 columns): one 128-column S buffer that the two tiles use in turn, P_0 and P_1
+// (64 columns each), O_0 and O_1 (128 each, fp32). A softmax group has S in registers some 250 clk
+// after it is complete; the buffer is then free for the other tile's S, and the next S of a tile is
+// ready before its group has finished the present one. (With P_t written over its own S_t a tile's
+// chain was S MMA -> softmax -> P V -> next S MMA, and the groups waited for S a third of the time:
+// 295 us at 4608 tokens x 32 heads, 278 us with the shared S buffer.)
+//
+// Issue order per key/value tile j:  S1_j, PV1_{j-1}, S0_{j+1}, PV0_j.
+//
+// What bounds it: the issuing warp shares its scheduler with two softmax warps, and per key tile it
+// needed some 3000 clk for what the tensor pipe does in 2048: 110 clk per barrier that was complete
+// anyway, 30 per MMA. Hence the looks ahead at barriers, one asm block and one elected lane per run of
+// MMAs, and operands the compiler knows to be uniform (278 -> 266 us). What is left is the
+// special-function unit, which the two groups share (2048 clk per key tile), and the power cap.
 //
 // Online softmax with a lazy reference maximum: the exponent reference of a row
 // only moves when some row of the warp sees a tile maximum more than 2^8 above it;
-// then the group rescales its O rows in TMEM itself. That window is safe because
-// the commit that published S_t for tile j also covers PV_t of tile j-1, and
-// PV_t of tile j is not issued before the group hands over P_t.
+// then the group rescales its O rows in TMEM itself, after the commit that says PV_t of tile j-1 is
+// complete; PV_t of tile j is not issued before the group hands over P_t.
 //
 // Arithmetic follows the reference flash kernel (F2K_CUDA
 // src/backend/cuda/attention.cu:601-757): scores scaled by `scale`, P rounded to
@@ -44,6 +54,8 @@
 
 #include <cuda_bf16.h>
 
+#include <type_traits>
+
 namespace f2k {
 
 using namespace f2k::ptx;
@@ -57,7 +69,7 @@ constexpr int kStages      = 4;
 constexpr uint32_t kTileBytes = kTileM * kHeadDim * 2;  // 32 KiB: one Q, K or V tile
 constexpr uint32_t kBoxBytes  = kTileBytes / 2;         // one 128 x 64 TMA box
 constexpr uint32_t kTmemCols  = 512;
-constexpr uint32_t kColS0 = 0, kColS1 = 128, kColO0 = 256, kColO1 = 384;
+constexpr uint32_t kColS = 0, kColP0 = 128, kColP1 = 192, kColO0 = 256, kColO1 = 384;
 constexpr float kLazyThreshold = 8.0f;  // log2 units
 
 // Tuning switches (compile-time; the defaults are what ships).
@@ -65,7 +77,7 @@ constexpr float kLazyThreshold = 8.0f;  // log2 units
 #define F2K_OPT_SETMAXNREG 1   // softmax warpgroups take registers from the load/MMA warpgroup
 #endif
 #ifndef F2K_OPT_P_PARTS
-#define F2K_OPT_P_PARTS 4      // P is handed to the MMA warp in this many parts (1, 2 or 4)
+#define F2K_OPT_P_PARTS 2      // P is handed to the MMA warp in this many parts (1, 2 or 4; 269, 266, 269 us at 4608 tokens x 32 heads)
 #endif
 #ifndef F2K_OPT_POLY_OF8
 #define F2K_OPT_POLY_OF8 0     // of every 8 key pairs, how many take 2^x on the FMA pipe (0..8); see softmax_row.cuh
@@ -84,8 +96,9 @@ struct SmemCtl {
     uint64_t kv_full[kStages];
     uint64_t kv_empty[kStages];
     uint64_t s_full[2];
+    uint64_t s_free;               // S has been read into registers: the other tile's S may be written
     uint64_t p_full[2][kPParts];   // [tile][part of the key tile]
-    uint64_t o_full[2];
+    uint64_t pv_done[2];           // P_t V_j is complete: P_t may be rewritten, O_t may be touched
     uint64_t drain;
     uint64_t xchg_full[2][2];      // head exchange: [warp][staging buffer] loaded
     uint32_t tmem_base;
@@ -110,36 +123,28 @@ __device__ __forceinline__ void locate_tile(const int* tile_start, const int* le
     valid = min(kTileN, len[seg] - row0);
 }
 
-// The MMA-issuing thread is a single lane that shares its scheduler with softmax warps, so every
-// instruction it needs per MMA delays the tensor pipe. Descriptors are therefore built once and
-// advanced by adding a compile-time constant to their low word (the start-address field counts
-// 16-byte units and never carries out of its 14 bits inside the CTA's shared memory).
+// The MMA-issuing warp shares its scheduler with two softmax warps, so every instruction it needs per
+// MMA delays the tensor pipe. A block of MMAs is therefore one asm statement with one elected lane, and
+// descriptors are built once and advanced by adding a compile-time constant (the start-address field
+// counts 16-byte units and never carries out of its 14 bits inside the CTA's shared memory).
 
 // S_t = Q_t K^T: 8 k-steps of 16 over head_dim; both operands K-major, 128-byte swizzle, stored as
 // two 128 x 64 boxes (k-steps 0-3 in the first, 4-7 in the second).
 __device__ __forceinline__ void issue_qk(uint32_t d_tmem, uint64_t q_desc, uint64_t k_desc) {
     constexpr uint32_t idesc = umma_idesc_bf16(kTileM, kTileN, /*b_mn_major=*/false);
-#pragma unroll
-    for (int kk = 0; kk < kHeadDim / 16; ++kk) {
-        constexpr uint32_t kBox16 = kBoxBytes >> 4;
-        const uint32_t off = (kk >> 2) * kBox16 + (kk & 3) * 2;   // in 16-byte units
-        umma_ss(d_tmem, q_desc + off, k_desc + off, idesc, kk > 0 ? 1u : 0u);
-    }
+    static_assert(kHeadDim == 128 && kBoxBytes == 16384, "the steps of umma_ss_x8");
+    umma_ss_x8(d_tmem, q_desc, k_desc, idesc);
 }
 
 // O_t (+)= P_t V: 8 k-steps of 16 keys. A = P_t in TMEM (two bf16 per 32-bit column, 8 columns per
 // k-step); B = V tile, MN-major: head_dim contiguous in 64-element (128-byte) swizzled rows, one
 // row per key, the second 64 head-dim elements one box (16 KiB) further on; 8-key groups are
-// 1024 bytes apart. `part` selects 8 / kPParts consecutive k-steps.
-__device__ __forceinline__ void issue_pv_part(uint32_t d_tmem, uint32_t p_tmem, uint64_t v_desc,
-                                              int part, uint32_t accumulate) {
+// 1024 bytes apart. kPart selects the k-steps.
+template <int kPart>
+__device__ __forceinline__ void issue_pv_part(uint32_t d_tmem, uint32_t p_tmem, uint64_t v_desc, uint32_t accumulate) {
     constexpr uint32_t idesc = umma_idesc_bf16(kTileM, kHeadDim, /*b_mn_major=*/true);
-    constexpr int kSteps = 8 / kPParts;
-#pragma unroll
-    for (int k4 = 0; k4 < kSteps; ++k4) {
-        const int kk = part * kSteps + k4;
-        umma_ts(d_tmem, p_tmem + kk * 8, v_desc + kk * (2048 >> 4), idesc, kk > 0 ? 1u : accumulate);
-    }
+    constexpr int kSteps = 8 / kPParts, kk = kPart * kSteps;
+    umma_ts_xn<kSteps>(d_tmem, p_tmem + kk * 8, v_desc + kk * (2048 >> 4), idesc, kPart > 0 ? 1u : accumulate);
 }
 
 // Head exchange by one of the CTA's two spare warps (see ExchangeParams). A chunk is 16 tokens of
@@ -297,7 +302,9 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
     SmemCtl* ctl = reinterpret_cast<SmemCtl*>(smem_raw + (smem - raw_addr) + kSmemCtl);
     volatile uint32_t* abort_flag = &ctl->abort;
 
-    const int warp = threadIdx.x >> 5;
+    // The shuffle tells the compiler that the role branches below are taken by whole warps: only then
+    // does it keep the MMA warp's descriptors in uniform registers.
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
     const int pair = p.grid_head_fastest ? blockIdx.y : blockIdx.x;
     const int head = p.grid_head_fastest ? blockIdx.x : blockIdx.y;
@@ -313,9 +320,10 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
         for (int i = 0; i < 2; ++i) {
             mbar_init(smem_u32(&ctl->q_full[i]), 1);
             mbar_init(smem_u32(&ctl->s_full[i]), 1);
-            for (int k = 0; k < kPParts; ++k) mbar_init(smem_u32(&ctl->p_full[i][k]), 128);
-            mbar_init(smem_u32(&ctl->o_full[i]), 1);
+            for (int k = 0; k < kPParts; ++k) mbar_init(smem_u32(&ctl->p_full[i][k]), 4);
+            mbar_init(smem_u32(&ctl->pv_done[i]), 1);
         }
+        mbar_init(smem_u32(&ctl->s_free), 4);
         for (int i = 0; i < kStages; ++i) {
             mbar_init(smem_u32(&ctl->kv_full[i]), 1);
             mbar_init(smem_u32(&ctl->kv_empty[i]), 1);
@@ -335,7 +343,10 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&ctl->tmem_base);
+    // All 512 columns are taken, so the allocation starts at column 0: a constant, which spares every
+    // tensor-memory address a register (checked: anything else ends the CTA with the status word set).
+    constexpr uint32_t tmem = 0;
+    if (*reinterpret_cast<volatile uint32_t*>(&ctl->tmem_base) != tmem) ctl->abort = 1;
 
     if (warp >= 8) {
         // ===================== warpgroup 2: TMA producer, MMA issuer, two idle warps =====================
@@ -434,61 +445,96 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
                 const uint32_t bar_full0 = smem_u32(&ctl->kv_full[0]), bar_empty0 = smem_u32(&ctl->kv_empty[0]);
                 // Ring slot of K_j is 2j, of V_j is 2j+1.
                 auto slot_off16 = [&](int n) { return (uint32_t)(n % kStages) * (kTileBytes >> 4); };
+                // A barrier that is already complete still costs the round trip of a try_wait, some
+                // 110 clk. Each wait is therefore looked at ahead (`peek`, before the MMAs in front of
+                // it are issued) and only waited for when the look found it incomplete. Two barriers
+                // are looked at in one instruction, half of the lanes each.
                 auto wait_uniform = [&](uint32_t bar, uint32_t parity) {
                     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, wait_limit)) != 0;
                 };
-                auto wait_full = [&](int n) {
-                    return wait_uniform(bar_full0 + (n % kStages) * 8, (n / kStages) & 1);
+                struct Look { uint32_t bar_a, par_a, bar_b, par_b; bool seen; };
+                auto peek2 = [&](uint32_t bar_a, uint32_t par_a, uint32_t bar_b, uint32_t par_b) {
+                    return Look{bar_a, par_a, bar_b, par_b, mbar_test(lane < 16 ? bar_a : bar_b, lane < 16 ? par_a : par_b)};
                 };
+                auto peek = [&](uint32_t bar, uint32_t par) { return Look{bar, par, bar, par, mbar_test(bar, par)}; };
+                auto finish = [&](const Look& l) {
+                    if (__all_sync(0xffffffffu, l.seen)) return true;
+                    return wait_uniform(l.bar_a, l.par_a) && (l.bar_b == l.bar_a || wait_uniform(l.bar_b, l.par_b));
+                };
+                auto bar_full = [&](int n) { return bar_full0 + (n % kStages) * 8; };
+                auto par_full = [&](int n) { return (uint32_t)(n / kStages) & 1u; };
                 auto release = [&](int n) { umma_commit(bar_empty0 + (n % kStages) * 8); };
-                // O_t (+)= P_t V_n, issued part by part as the softmax group hands P over.
-                auto issue_pv = [&](int t, int jj) -> bool {
+                const uint32_t bar_free = smem_u32(&ctl->s_free);
+                auto bar_p = [&](int t, int part) { return smem_u32(&ctl->p_full[t][part]); };
+                // S = Q_t K_j^T, and its commit.
+                auto issue_s = [&](int t, int jj) {
+                    tc_fence_after_sync();
+                    issue_qk(tmem + kColS, t == 0 ? q0_desc : q1_desc, k_desc0 + slot_off16(2 * jj));
+                    umma_commit(smem_u32(&ctl->s_full[t]));
+                };
+                // O_t (+)= P_t V_jj, issued part by part as the softmax group hands P over; `first` is
+                // the look at the first part (and V). The look at the barriers behind it is taken by
+                // `next`, in front of the last part's MMAs.
+                auto issue_pv = [&](int t, int jj, const Look& first, auto&& next) -> bool {
                     const uint32_t d = tmem + (t == 0 ? kColO0 : kColO1);
-                    const uint32_t a = tmem + (t == 0 ? kColS0 : kColS1);
+                    const uint32_t a = tmem + (t == 0 ? kColP0 : kColP1);
                     const uint64_t v_desc = v_desc0 + slot_off16(2 * jj + 1);
-                    const uint32_t bar_p = smem_u32(&ctl->p_full[t][0]);
-#pragma unroll
-                    for (int part = 0; part < kPParts; ++part) {
-                        if (!wait_uniform(bar_p + part * 8, jj & 1)) return false;
+                    if (!finish(first)) return false;
+                    auto rest = [&](auto self, auto part) -> bool {
+                        constexpr int kPart = decltype(part)::value;
+                        Look look{};
+                        if constexpr (kPart + 1 < kPParts) look = peek(bar_p(t, kPart + 1), jj & 1);
+                        else next();
                         tc_fence_after_sync();
-                        issue_pv_part(d, a, v_desc, part, jj > 0 ? 1u : 0u);
-                    }
+                        issue_pv_part<kPart>(d, a, v_desc, jj > 0 ? 1u : 0u);
+                        if constexpr (kPart + 1 < kPParts) {
+                            if (!finish(look)) return false;
+                            return self(self, std::integral_constant<int, kPart + 1>{});
+                        }
+                        return true;
+                    };
+                    if (!rest(rest, std::integral_constant<int, 0>{})) return false;
+                    umma_commit(smem_u32(&ctl->pv_done[t]));
                     return true;
                 };
 
-                for (int j = 0; j < n_kv; ++j) {
-                    // S0_j
-                    if (!(ok = wait_full(2 * j))) break;
-                    if (j == 0 && !(ok = wait_uniform(smem_u32(&ctl->q_full[0]), 0))) break;
-                    tc_fence_after_sync();
-                    issue_qk(tmem + kColS0, q0_desc, k_desc0 + slot_off16(2 * j));
-                    umma_commit(smem_u32(&ctl->s_full[0]));
+                // The S buffer is used in turn: use number u waits for release number u - 1. With two
+                // tiles S0_j is use 2j and S1_j use 2j + 1, with one S0_j is use j.
+                Look look_s{}, look_p{};
+                if (n_kv > 0) {
+                    ok = wait_uniform(bar_full(0), par_full(0)) && wait_uniform(smem_u32(&ctl->q_full[0]), 0);
+                    if (ok) issue_s(0, 0);
+                    if (ok && has_t1) ok = wait_uniform(smem_u32(&ctl->q_full[1]), 0);
+                    look_s = peek(bar_free, 0);
+                }
+                for (int j = 0; j < n_kv && ok; ++j) {
                     if (has_t1) {
-                        // PV1_{j-1}
-                        if (j > 0) {
-                            if (!(ok = issue_pv(1, j - 1))) break;
-                            release(2 * j - 1);
-                        }
-                        // S1_j
-                        if (j == 0 && !(ok = wait_uniform(smem_u32(&ctl->q_full[1]), 0))) break;
-                        tc_fence_after_sync();
-                        issue_qk(tmem + kColS1, q1_desc, k_desc0 + slot_off16(2 * j));
-                        umma_commit(smem_u32(&ctl->s_full[1]));
+                        if (!(ok = finish(look_s))) break;                       // S0_j is in registers
+                        if (j > 0) look_p = peek(bar_p(1, 0), (j - 1) & 1);
+                        issue_s(1, j);
                     }
                     release(2 * j);
-                    // PV0_j
-                    if (!(ok = wait_full(2 * j + 1))) break;
-                    if (!(ok = issue_pv(0, j))) break;
+                    auto look_next_s0 = [&] {
+                        if (j + 1 < n_kv)
+                            look_s = peek2(bar_full(2 * j + 2), par_full(2 * j + 2), bar_free, has_t1 ? 1u : (uint32_t)(j & 1));
+                    };
+                    if (has_t1 && j > 0) {
+                        if (!(ok = issue_pv(1, j - 1, look_p, look_next_s0))) break;
+                        release(2 * j - 1);
+                    } else {
+                        look_next_s0();
+                    }
+                    if (j + 1 < n_kv) {
+                        if (!(ok = finish(look_s))) break;                       // K_{j+1}; S1_j is in registers
+                    }
+                    look_p = peek2(bar_full(2 * j + 1), par_full(2 * j + 1), bar_p(0, 0), j & 1);
+                    if (j + 1 < n_kv) issue_s(0, j + 1);
+                    if (!(ok = issue_pv(0, j, look_p, [&] { if (has_t1) look_s = peek(bar_free, 0); }))) break;
                     if (!has_t1) release(2 * j + 1);
-                    if (j == n_kv - 1) umma_commit(smem_u32(&ctl->o_full[0]));
                 }
                 if (ok && n_kv > 0 && has_t1) {
-                    // PV1 of the last tile
-                    ok = issue_pv(1, n_kv - 1);
-                    if (ok) {
-                        release(2 * n_kv - 1);
-                        umma_commit(smem_u32(&ctl->o_full[1]));
-                    }
+                    ok = issue_pv(1, n_kv - 1, peek(bar_p(1, 0), (n_kv - 1) & 1), [] {});
+                    if (ok) release(2 * n_kv - 1);
                 }
                 if (!ok) {
                     // Leaving early: wait (bounded) until the MMAs already issued retire, so
@@ -507,7 +553,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
 #endif
         const int t = warp >> 2;                                       // which query tile
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;  // this warp's TMEM lanes
-        const uint32_t tS = tmem + lane_base + (t == 0 ? kColS0 : kColS1);
+        const uint32_t tS = tmem + lane_base + kColS;
+        const uint32_t tP = tmem + lane_base + (t == 0 ? kColP0 : kColP1);
         const uint32_t tO = tmem + lane_base + (t == 0 ? kColO0 : kColO1);
         const float c = p.scale_log2;
 
@@ -548,6 +595,9 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
                 }
                 row_max64<true>(&s[0], mx);
                 tmem_wait_ld();
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&ctl->s_free));
             }
             if (valid < kTileN) {
 #pragma unroll
@@ -556,6 +606,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
             }
             row_max64<false>(&s[64], mx);
             const float m_tile = row_max_finish(mx);
+            // looked at here, needed a few hundred clocks later
+            const bool pv_seen = j == 0 || mbar_test(smem_u32(&ctl->pv_done[t]), (j - 1) & 1);
 
             const bool need = (m_tile - m_ref) * c > kLazyThreshold;
             if (__any_sync(0xffffffffu, need)) {
@@ -564,7 +616,11 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
                 l_sum *= f;
                 m_ref = m_new;
                 if (j > 0) {
-                    // Rescale this row of O in place (O_t is idle, see the file header).
+                    // Rescale this row of O in place, once P V of the previous key tile is in.
+                    ok = mbar_wait(smem_u32(&ctl->pv_done[t]), (j - 1) & 1, abort_flag, wait_limit);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    tc_fence_after_sync();
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         uint32_t o[32];
@@ -592,22 +648,31 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
                 if (pending >= 0) {
                     tmem_wait_st();
                     tc_fence_before_sync();
-                    mbar_arrive(smem_u32(&ctl->p_full[t][0]) + pending * 8);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&ctl->p_full[t][0]) + pending * 8);
                     pending = -1;
                 }
                 exp_chunk16<F2K_OPT_POLY_OF8>(&s[q * 32 + 16], pk + 8, c, neg_mc, sum);
-                tmem_st_x16(tS + q * 16, pk);
+                if (q == 0 && !__all_sync(0xffffffffu, pv_seen)) {   // P_t of the previous key tile is still being read
+                    ok = mbar_wait(smem_u32(&ctl->pv_done[t]), (j - 1) & 1, abort_flag, wait_limit);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                }
+                if (q == 0) tc_fence_after_sync();
+                tmem_st_x16(tP + q * 16, pk);
                 if ((q + 1) % (4 / kPParts) == 0) pending = (q + 1) / (4 / kPParts) - 1;
             }
+            if (!ok) break;
             tmem_wait_st();
             tc_fence_before_sync();
-            mbar_arrive(smem_u32(&ctl->p_full[t][kPParts - 1]));
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&ctl->p_full[t][kPParts - 1]));
             l_sum += (sum[0] + sum[1]) + (sum[2] + sum[3]);
         }
 
         // ------------------------------ epilogue ------------------------------------
         if (ok && n_iter > 0) {
-            ok = mbar_wait(smem_u32(&ctl->o_full[t]), 0, abort_flag, wait_limit);
+            ok = mbar_wait(smem_u32(&ctl->pv_done[t]), (n_iter - 1) & 1, abort_flag, wait_limit);
             ok = __all_sync(0xffffffffu, ok);
         }
         if (ok && n_iter > 0) {

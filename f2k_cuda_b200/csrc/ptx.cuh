@@ -48,6 +48,21 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 
+// One look, without waiting: is the phase of this parity complete?
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred P;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, P;\n\t"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
 // Bounded wait. `abort_flag` is a CTA-shared word any role sets when it gives up;
 // it is polled so that one expired wait releases every other waiter quickly.
 // Returns false when the limit ran out or the CTA is aborting. The limit is kept on the
@@ -262,35 +277,77 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n, bool b_mn_m
 // (A divergent single-lane branch would force the operands out of the uniform datapath and cost
 // tens of cycles per MMA on a warp that shares its scheduler with the softmax warps.)
 
-// D[tmem] (+)= A[smem] * B[smem]
-__device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                        uint32_t idesc, uint32_t accumulate) {
+// D[tmem] = A[smem] * B[smem] over 8 k-steps of 16 elements: descriptors advance by 2 (32 bytes) inside
+// a 128-byte swizzled row of 64 elements, and by 1024 (16 KiB) to the second box of 64.
+__device__ __forceinline__ void umma_ss_x8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
     asm volatile(
         "{\n\t"
-        ".reg .pred pe, p;\n\t"
+        ".reg .pred pe, fresh, more;\n\t"
+        ".reg .b64 a, b;\n\t"
         "elect.sync _|pe, 0xffffffff;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "setp.ne.b32 fresh, 0, 0;\n\t"
+        "setp.eq.b32 more, 0, 0;\n\t"
+        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, fresh;\n\t"
+        "add.s64 a, %1, 2;\n\t"
+        "add.s64 b, %2, 2;\n\t"
+        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, more;\n\t"
+        "add.s64 a, %1, 4;\n\t"
+        "add.s64 b, %2, 4;\n\t"
+        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, more;\n\t"
+        "add.s64 a, %1, 6;\n\t"
+        "add.s64 b, %2, 6;\n\t"
+        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, more;\n\t"
+        "add.s64 a, %1, 1024;\n\t"
+        "add.s64 b, %2, 1024;\n\t"
+        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, more;\n\t"
+        "add.s64 a, %1, 1026;\n\t"
+        "add.s64 b, %2, 1026;\n\t"
+        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, more;\n\t"
+        "add.s64 a, %1, 1028;\n\t"
+        "add.s64 b, %2, 1028;\n\t"
+        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, more;\n\t"
+        "add.s64 a, %1, 1030;\n\t"
+        "add.s64 b, %2, 1030;\n\t"
+        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, more;\n\t"
         "}\n"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc)
         : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem]
-__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
-                                        uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred pe, p;\n\t"
-        "elect.sync _|pe, 0xffffffff;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-        "}\n"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
+// D[tmem] (+)= A[tmem] * B[smem] over kSteps k-steps of 16: 8 columns of A and 2048 bytes of B each.
+#define F2K_UMMA_TS_STEP(K)                                  \
+    "add.s32 a, %1, " #K " * 8;\n\t"                         \
+    "add.s64 b, %2, " #K " * 128;\n\t"                       \
+    "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, more;\n\t"
+#define F2K_UMMA_TS(STEPS)                                                                   \
+    asm volatile(                                                                            \
+        "{\n\t"                                                                              \
+        ".reg .pred pe, p, more;\n\t"                                                        \
+        ".reg .b32 a;\n\t"                                                                   \
+        ".reg .b64 b;\n\t"                                                                   \
+        "elect.sync _|pe, 0xffffffff;\n\t"                                                   \
+        "setp.ne.b32 p, %4, 0;\n\t"                                                          \
+        "setp.eq.b32 more, 0, 0;\n\t"                                                        \
+        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t" STEPS            \
+        "}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory")
+template <int kSteps>
+__device__ __forceinline__ void umma_ts_xn(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                           uint32_t accumulate) {
+    static_assert(kSteps == 2 || kSteps == 4 || kSteps == 6 || kSteps == 8, "written out below");
+    if constexpr (kSteps == 2)
+        F2K_UMMA_TS(F2K_UMMA_TS_STEP(1));
+    else if constexpr (kSteps == 4)
+        F2K_UMMA_TS(F2K_UMMA_TS_STEP(1) F2K_UMMA_TS_STEP(2) F2K_UMMA_TS_STEP(3));
+    else if constexpr (kSteps == 6)
+        F2K_UMMA_TS(F2K_UMMA_TS_STEP(1) F2K_UMMA_TS_STEP(2) F2K_UMMA_TS_STEP(3) F2K_UMMA_TS_STEP(4) F2K_UMMA_TS_STEP(5));
+    else
+        F2K_UMMA_TS(F2K_UMMA_TS_STEP(1) F2K_UMMA_TS_STEP(2) F2K_UMMA_TS_STEP(3) F2K_UMMA_TS_STEP(4) F2K_UMMA_TS_STEP(5)
+                    F2K_UMMA_TS_STEP(6) F2K_UMMA_TS_STEP(7));
 }
+#undef F2K_UMMA_TS
+#undef F2K_UMMA_TS_STEP
 // Arrive (count 1) on `bar` once every tcgen05 operation the elected lane issued before the
 // commit has completed. elect.sync picks the same lane every time for a full warp, so the
-// commit tracks the MMAs issued through umma_ss / umma_ts.
+// commit tracks the MMAs issued through umma_ss_x8 / umma_ts_xn.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile(
         "{\n\t"
