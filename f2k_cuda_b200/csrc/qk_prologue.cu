@@ -47,24 +47,30 @@ __device__ __forceinline__ float warp_sum(float v) {
 template <int kGroup>
 __global__ void __launch_bounds__(kBlock, 4)
 qk_prologue_kernel(const __grid_constant__ QkPrologueParams p) {
+    // The attention kernel behind this one may set itself up while this one drains; and this one may
+    // have started before the kernel in front of it has ended.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int hl = threadIdx.x & 15;  // lane inside the half-warp
-    const long long total = p.row_start[p.n_jobs] / kGroup;          // in groups
-    const long long n_hw  = (long long)gridDim.x * (kBlock / 16);
-    for (long long grp = (long long)blockIdx.x * (kBlock / 16) + (threadIdx.x >> 4); grp < total; grp += n_hw) {
-        const long long row = grp * kGroup;
+    // Row numbers fit 32 bits (2^31 rows of 256 bytes exceed any memory; the launch checks it): two
+    // 64-bit divisions per group of rows took more instructions than the arithmetic.
+    const unsigned total = (unsigned)p.row_start[p.n_jobs] / kGroup;          // in groups
+    const unsigned n_hw  = gridDim.x * (kBlock / 16);
+    for (unsigned grp = blockIdx.x * (kBlock / 16) + (threadIdx.x >> 4); grp < total; grp += n_hw) {
+        const unsigned row = grp * kGroup;
         int j = 0;
 #pragma unroll
         for (int i = 1; i < kMaxPrologueJobs; ++i)
-            if (i < p.n_jobs && row >= p.row_start[i]) j = i;
+            if (i < p.n_jobs && row >= (unsigned)p.row_start[i]) j = i;
         const QkPrologueJob& job = p.job[j];
-        const long long lr = row - p.row_start[j];
-        const long long trow = lr / p.n_heads;                 // token row over batch * seq
-        const int tok = (int)(trow % job.seq);
-        const int hd0 = (int)(lr - trow * p.n_heads);           // first head of the group
+        const unsigned lr = row - (unsigned)p.row_start[j];
+        const unsigned trow = lr / (unsigned)p.n_heads;         // token row over batch * seq
+        const unsigned tok = trow % (unsigned)job.seq;
+        const unsigned hd0 = lr - trow * (unsigned)p.n_heads;   // first head of the group
         // plain loads of x: y may alias x, so x is not read-only for the kernel's lifetime. A token
         // row of x may be a slice of a wider row (x_tok_stride); y is always dense.
         const uint4* src = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(job.x) +
-                                                          trow * job.x_tok_stride + (long long)hd0 * kHeadDim);
+                                                          (long long)trow * job.x_tok_stride + hd0 * kHeadDim);
         uint4 raw[kGroup];
 #pragma unroll
         for (int u = 0; u < kGroup; ++u) raw[u] = src[u * 16 + hl];
@@ -75,25 +81,9 @@ qk_prologue_kernel(const __grid_constant__ QkPrologueParams p) {
         unpack8(graw, g);
         const float cs[4] = {c4.x, c4.y, c4.z, c4.w};
         const float sn[4] = {s4.x, s4.y, s4.z, s4.w};
-        uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(job.y) + lr * kHeadDim);
+        uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(job.y) + (long long)lr * kHeadDim);
 #pragma unroll
-        for (int u = 0; u < kGroup; ++u) {
-            float v[8];
-            unpack8(raw[u], v);
-            float ss = 0.f;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) ss = fmaf(v[i], v[i], ss);
-            ss = half_warp_sum(ss);
-            const float rrms = rsqrtf(ss * (1.0f / kHeadDim) + p.eps);
-            float y[8];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const float a = v[2 * k] * rrms * g[2 * k];
-                const float b = v[2 * k + 1] * rrms * g[2 * k + 1];
-                rotate_pair(y[2 * k], y[2 * k + 1], a, b, cs[k], sn[k]);
-            }
-            dst[u * 16 + hl] = pack8(y);
-        }
+        for (int u = 0; u < kGroup; ++u) dst[u * 16 + hl] = norm_rope_row(raw[u], g, cs, sn, p.eps);
     }
 }
 
@@ -173,30 +163,43 @@ qkv_scatter_kernel(const __grid_constant__ QkvScatterParams p) {
 // ---------------------------------------------------------------------------------
 // Stand-alone RMSNorm. dim == 128: half-warp per row, one pass. Other dims (multiple
 // of 8): one warp per row, two passes over the row (the second hits L1/L2).
+// A half-warp takes kRowsAhead consecutive rows at a time, their loads issued back to back: one row
+// at a time is bound by the latency of one 16-byte load per lane.
 // y = bf16( x * rsqrt(mean(x^2) + eps) * gamma ), fp32 arithmetic.
 // ---------------------------------------------------------------------------------
+constexpr int kRowsAhead = 4;
+
 __global__ void __launch_bounds__(kBlock)
 rmsnorm_rows128_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ gamma,
                        __nv_bfloat16* y, long long rows, float eps) {  // y may alias x
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int hl = threadIdx.x & 15;
     const long long n_hw = (long long)gridDim.x * (kBlock / 16);
     const uint4 graw = __ldg(reinterpret_cast<const uint4*>(gamma) + hl);
     float g[8];
     unpack8(graw, g);
-    for (long long row = (long long)blockIdx.x * (kBlock / 16) + (threadIdx.x >> 4); row < rows;
-         row += n_hw) {
-        const uint4 raw = reinterpret_cast<const uint4*>(x + row * 128)[hl];
-        float v[8];
-        unpack8(raw, v);
-        float ss = 0.f;
+    for (long long row0 = ((long long)blockIdx.x * (kBlock / 16) + (threadIdx.x >> 4)) * kRowsAhead; row0 < rows;
+         row0 += n_hw * kRowsAhead) {
+        uint4 raw[kRowsAhead];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) ss = fmaf(v[i], v[i], ss);
-        ss = half_warp_sum(ss);
-        const float rrms = rsqrtf(ss * (1.0f / 128.0f) + eps);
-        float o[8];
+        for (int u = 0; u < kRowsAhead; ++u)
+            if (row0 + u < rows) raw[u] = reinterpret_cast<const uint4*>(x + (row0 + u) * 128)[hl];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = v[i] * rrms * g[i];
-        reinterpret_cast<uint4*>(y + row * 128)[hl] = pack8(o);
+        for (int u = 0; u < kRowsAhead; ++u) {
+            if (row0 + u >= rows) break;                     // the same for the whole half-warp
+            float v[8];
+            unpack8(raw[u], v);
+            float ss = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) ss = fmaf(v[i], v[i], ss);
+            ss = half_warp_sum(ss);
+            const float rrms = rsqrtf(ss * (1.0f / 128.0f) + eps);
+            float o[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = v[i] * rrms * g[i];
+            reinterpret_cast<uint4*>(y + (row0 + u) * 128)[hl] = pack8(o);
+        }
     }
 }
 
@@ -239,22 +242,37 @@ __global__ void __launch_bounds__(kBlock)
 rope4_rows128_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ cos_tab,
                      const float* __restrict__ sin_tab, const int32_t* __restrict__ pos_ids,
                      long long rows, int seq_max) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int hl = threadIdx.x & 15;
     const long long n_hw = (long long)gridDim.x * (kBlock / 16);
-    for (long long row = (long long)blockIdx.x * (kBlock / 16) + (threadIdx.x >> 4); row < rows;
-         row += n_hw) {
-        int pos = __ldg(pos_ids + row);
-        pos = pos >= seq_max ? seq_max - 1 : (pos < 0 ? 0 : pos);
-        uint4* xp = reinterpret_cast<uint4*>(x + row * 128) + hl;
-        const float4 c4 = __ldg(reinterpret_cast<const float4*>(cos_tab + (long long)pos * 64) + hl);
-        const float4 s4 = __ldg(reinterpret_cast<const float4*>(sin_tab + (long long)pos * 64) + hl);
-        float v[8], o[8];
-        unpack8(*xp, v);
-        const float cs[4] = {c4.x, c4.y, c4.z, c4.w};
-        const float sn[4] = {s4.x, s4.y, s4.z, s4.w};
+    for (long long row0 = ((long long)blockIdx.x * (kBlock / 16) + (threadIdx.x >> 4)) * kRowsAhead; row0 < rows;
+         row0 += n_hw * kRowsAhead) {
+        uint4 raw[kRowsAhead];
+        int pos[kRowsAhead];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) rotate_pair(o[2 * k], o[2 * k + 1], v[2 * k], v[2 * k + 1], cs[k], sn[k]);
-        *xp = pack8(o);
+        for (int u = 0; u < kRowsAhead; ++u)
+            if (row0 + u < rows) {
+                raw[u] = reinterpret_cast<const uint4*>(x + (row0 + u) * 128)[hl];
+                const int pid = __ldg(pos_ids + row0 + u);
+                pos[u] = pid >= seq_max ? seq_max - 1 : (pid < 0 ? 0 : pid);
+            }
+        float4 c4, s4;
+#pragma unroll
+        for (int u = 0; u < kRowsAhead; ++u) {
+            if (row0 + u >= rows) break;
+            if (u == 0 || pos[u] != pos[u - 1]) {            // the heads of one token share a table row
+                c4 = __ldg(reinterpret_cast<const float4*>(cos_tab + (long long)pos[u] * 64) + hl);
+                s4 = __ldg(reinterpret_cast<const float4*>(sin_tab + (long long)pos[u] * 64) + hl);
+            }
+            float v[8], o[8];
+            unpack8(raw[u], v);
+            const float cs[4] = {c4.x, c4.y, c4.z, c4.w};
+            const float sn[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) rotate_pair(o[2 * k], o[2 * k + 1], v[2 * k], v[2 * k + 1], cs[k], sn[k]);
+            reinterpret_cast<uint4*>(x + (row0 + u) * 128)[hl] = pack8(o);
+        }
     }
 }
 
@@ -297,6 +315,22 @@ int grid_for(long long units, int units_per_block) {
     return (int)(need < cap ? (need > 0 ? need : 1) : cap);
 }
 
+// A launch that may start while the kernel in front of it drains; the kernel itself waits for that one's
+// end before it touches memory.
+template <typename... P, typename... A>
+cudaError_t launch_overlapping(void (*kernel)(P...), int grid, cudaStream_t stream, A&&... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kBlock);
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 }  // namespace
 
 cudaError_t qk_prologue_prepare() {
@@ -314,11 +348,9 @@ cudaError_t qk_prologue_launch(const QkPrologueParams& params, cudaStream_t stre
         if (p.job[i].x_tok_stride == 0) p.job[i].x_tok_stride = (long long)p.n_heads * kHeadDim;
     const long long total = p.row_start[p.n_jobs];
     if (total <= 0) return cudaSuccess;
-    if (p.n_heads % 4 == 0)
-        qk_prologue_kernel<4><<<grid_for(total / 4, kBlock / 16), kBlock, 0, stream>>>(p);
-    else
-        qk_prologue_kernel<1><<<grid_for(total, kBlock / 16), kBlock, 0, stream>>>(p);
-    return cudaPeekAtLastError();
+    if (total >= 1ll << 31) return cudaErrorInvalidValue;
+    if (p.n_heads % 4 == 0) return launch_overlapping(qk_prologue_kernel<4>, grid_for(total / 4, kBlock / 16), stream, p);
+    return launch_overlapping(qk_prologue_kernel<1>, grid_for(total, kBlock / 16), stream, p);
 }
 
 cudaError_t qkv_scatter_launch(const QkvScatterParams& p, cudaStream_t stream) {
@@ -337,7 +369,8 @@ cudaError_t rmsnorm_rows_launch(const void* x, const void* gamma, void* y, int r
     auto gb = static_cast<const __nv_bfloat16*>(gamma);
     auto yb = static_cast<__nv_bfloat16*>(y);
     if (dim == 128) {
-        rmsnorm_rows128_kernel<<<grid_for(rows, kBlock / 16), kBlock, 0, stream>>>(xb, gb, yb, rows, eps);
+        return launch_overlapping(rmsnorm_rows128_kernel, grid_for(rows, kBlock / 16 * kRowsAhead), stream, xb, gb, yb,
+                                  (long long)rows, eps);
     } else {
         rmsnorm_rows_generic_kernel<<<grid_for(rows, kBlock / 32), kBlock, 0, stream>>>(
             xb, gb, yb, rows, dim, 1.0f / (float)dim, eps);
@@ -350,8 +383,8 @@ cudaError_t rope4_rows_launch(void* x, const float* cos_tab, const float* sin_ta
                               cudaStream_t stream) {
     auto xb = static_cast<__nv_bfloat16*>(x);
     if (head_dim == 128) {
-        rope4_rows128_kernel<<<grid_for(rows, kBlock / 16), kBlock, 0, stream>>>(xb, cos_tab, sin_tab,
-                                                                                pos_ids, rows, seq_max);
+        return launch_overlapping(rope4_rows128_kernel, grid_for(rows, kBlock / 16 * kRowsAhead), stream, xb, cos_tab,
+                                  sin_tab, pos_ids, (long long)rows, seq_max);
     } else {
         rope4_rows_generic_kernel<<<grid_for(rows, kBlock / 32), kBlock, 0, stream>>>(
             xb, cos_tab, sin_tab, pos_ids, rows, head_dim, seq_max);
