@@ -306,17 +306,53 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
     // does it keep the MMA warp's descriptors in uniform registers.
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
-    const int pair = p.grid_head_fastest ? blockIdx.y : blockIdx.x;
-    const int head = p.grid_head_fastest ? blockIdx.x : blockIdx.y;
-    const int bidx = blockIdx.z;
     const int n_kv = p.n_kv_tiles;
-    // With an odd number of query tiles the last CTA of a (batch, head) has one tile only: its
-    // second softmax group, and the MMAs that would feed it, are left out.
-    const bool has_t1 = 2 * pair + 1 < p.n_q_tiles;
+    // This CTA's query tiles: qt0 and, with has_t1, qt0 + 1. A CTA with one tile leaves its second
+    // softmax group, and the MMAs that would feed it, out.
+    int qt0, head, bidx;
+    bool has_t1;
+    if (p.grid_head_fastest) {
+        qt0 = 2 * blockIdx.y;
+        head = blockIdx.x;
+        bidx = blockIdx.z;
+        has_t1 = qt0 + 1 < p.n_q_tiles;
+    } else {
+        const CtaWork w = cta_work(p.plan, p.n_q_tiles, (int)blockIdx.x);
+        qt0 = w.tile;
+        has_t1 = w.two;
+        bidx = w.group / p.n_heads;
+        head = w.group - bidx * p.n_heads;
+    }
     const long long peer_limit = p.peer_wait_limit_clk;
     const long long wait_limit = p.wait_limit_clk;
 
-    if (threadIdx.x == 0) {
+    // Loader state: it starts its copies as soon as its barriers exist, before the CTA-wide barrier
+    // below, unless a segment may still have to be waited for (the exchange's warps must run then).
+    int issued = 0, q_issued = 0;
+    auto load_q = [&](int t) {
+        int seg, row0, valid;
+        locate_tile<kMaxQSeg>(p.q_tile_start, p.q_len, p.n_qseg, qt0 + t, seg, row0, valid);
+        const uint32_t bar = smem_u32(&ctl->q_full[t]);
+        const uint32_t dst = smem + kSmemQ + t * kTileBytes;
+        mbar_arrive_expect_tx(bar, kTileBytes);
+        tma_load_4d(dst, &p.tm_q[seg], bar, 0, head, row0, bidx);
+        tma_load_4d(dst + kBoxBytes, &p.tm_q[seg], bar, 64, head, row0, bidx);
+        ++q_issued;
+    };
+    auto load_kv = [&](int seg, int row0, int kv) {          // into the next ring slot
+        const int slot = issued % kStages;
+        const uint32_t bar = smem_u32(&ctl->kv_full[slot]);
+        const uint32_t dst = smem + kSmemRing + slot * kTileBytes;
+        const CUtensorMap* tm = kv == 0 ? &p.tm_k[seg] : &p.tm_v[seg];
+        mbar_arrive_expect_tx(bar, kTileBytes);
+        tma_load_4d(dst, tm, bar, 0, head, row0, bidx);
+        tma_load_4d(dst + kBoxBytes, tm, bar, 64, head, row0, bidx);
+        ++issued;
+    };
+    // Once every CTA has started, the kernel behind this one may be set up on the SMs that are free. Not
+    // while this one may wait for another rank: where ranks share a GPU, that rank needs those SMs.
+    if (!kWithExchange && !p.waits_for_words) grid_launch_dependents();
+    if (warp == kLoaderWarp && lane == 0) {
         for (int i = 0; i < 2; ++i) {
             mbar_init(smem_u32(&ctl->q_full[i]), 1);
             mbar_init(smem_u32(&ctl->s_full[i]), 1);
@@ -335,6 +371,18 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
         ctl->softmax_done = 0;
         fence_mbar_init();
         fence_proxy_async_smem();
+        // Everything this kernel reads or overwrites may come from the kernel launched before it
+        // (programmatic dependent launch: this one may have started while that one drained).
+        grid_dependency_wait();
+        if (!p.waits_for_words) {
+            load_q(0);
+            for (int i = 0; i < min(kStages, 2 * n_kv); ++i) {
+                int seg, row0, valid;
+                locate_tile<kMaxKvSeg>(p.kv_tile_start, p.kv_len, p.n_kvseg, i >> 1, seg, row0, valid);
+                load_kv(seg, row0, i & 1);
+                if (i == 0 && has_t1) load_q(1);
+            }
+        }
     }
     if (warp == kMmaWarp) {
         tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols);
@@ -356,13 +404,10 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
         if (warp == kLoaderWarp) {
             // ------------------------------ TMA producer ------------------------------
             if (lane == 0) {
-                int issued = 0, q_issued = 0;
                 bool ok = true;
-                for (int t = 0; t < 2 && ok; ++t) {
-                    const int qt = 2 * pair + t;
-                    if (qt >= p.n_q_tiles) break;   // odd tile count: the last CTA of a head has one tile
+                for (int t = q_issued; t < (has_t1 ? 2 : 1) && ok; ++t) {
                     int seg, row0, valid;
-                    locate_tile<kMaxQSeg>(p.q_tile_start, p.q_len, p.n_qseg, qt, seg, row0, valid);
+                    locate_tile<kMaxQSeg>(p.q_tile_start, p.q_len, p.n_qseg, qt0 + t, seg, row0, valid);
                     if (p.q_ready[seg] != nullptr) {   // the segment is written by another GPU's kernel
                         ok = p.ready_per_tile
                                  ? global_flag_wait(p.q_ready[seg] + row0 / kTileM,
@@ -372,24 +417,20 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
                         if (!ok) break;
                         asm volatile("fence.proxy.async.global;" ::: "memory");
                     }
-                    const uint32_t bar = smem_u32(&ctl->q_full[t]);
-                    const uint32_t dst = smem + kSmemQ + t * kTileBytes;
-                    mbar_arrive_expect_tx(bar, kTileBytes);
-                    tma_load_4d(dst, &p.tm_q[seg], bar, 0, head, row0, bidx);
-                    tma_load_4d(dst + kBoxBytes, &p.tm_q[seg], bar, 64, head, row0, bidx);
-                    ++q_issued;
+                    load_q(t);
                 }
-                for (int j = 0; j < n_kv && ok; ++j) {
+                while (ok && issued < 2 * n_kv) {
+                    const int j = issued >> 1, kv = issued & 1;
                     int seg, row0, valid;
                     locate_tile<kMaxKvSeg>(p.kv_tile_start, p.kv_len, p.n_kvseg, j, seg, row0, valid);
-                    if (p.ready_per_tile && p.kv_ready[seg] != nullptr) {
+                    if (kv == 0 && p.ready_per_tile && p.kv_ready[seg] != nullptr) {
                         // fused head exchange: every tile has its own counter of delivered chunks
                         ok = global_flag_wait(p.kv_ready[seg] + row0 / kTileN,
                                               p.ready_uses * (unsigned)((valid + kExchangeTokens - 1) / kExchangeTokens),
                                               abort_flag, peer_limit);
                         if (!ok) break;
                         asm volatile("fence.proxy.async.global;" ::: "memory");
-                    } else if (row0 == 0 && p.kv_ready[seg] != nullptr) {
+                    } else if (kv == 0 && row0 == 0 && p.kv_ready[seg] != nullptr) {
                         // first tile of a segment that is being copied in: wait for its arrival word,
                         // then order the copy engine's writes before this thread's TMA reads
                         const unsigned int* word = p.kv_ready[seg] + head / max(1, p.kv_ready_heads_per_group);
@@ -398,20 +439,9 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
                         if (!ok) break;
                         asm volatile("fence.proxy.async.global;" ::: "memory");
                     }
-#pragma unroll
-                    for (int kv = 0; kv < 2; ++kv) {
-                        const int slot = issued % kStages;
-                        const uint32_t par = (issued / kStages) & 1;
-                        ok = mbar_wait(smem_u32(&ctl->kv_empty[slot]), par ^ 1u, abort_flag, wait_limit);
-                        if (!ok) break;
-                        const uint32_t bar = smem_u32(&ctl->kv_full[slot]);
-                        const uint32_t dst = smem + kSmemRing + slot * kTileBytes;
-                        const CUtensorMap* tm = kv == 0 ? &p.tm_k[seg] : &p.tm_v[seg];
-                        mbar_arrive_expect_tx(bar, kTileBytes);
-                        tma_load_4d(dst, tm, bar, 0, head, row0, bidx);
-                        tma_load_4d(dst + kBoxBytes, tm, bar, 64, head, row0, bidx);
-                        ++issued;
-                    }
+                    ok = mbar_wait(smem_u32(&ctl->kv_empty[issued % kStages]), ((issued / kStages) & 1) ^ 1u, abort_flag,
+                                   wait_limit);
+                    if (ok) load_kv(seg, row0, kv);
                 }
                 if (!ok) {
                     // Leaving early: let the copies this thread started land first.
@@ -677,7 +707,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
         }
         if (ok && n_iter > 0) {
             tc_fence_after_sync();
-            const int qt = 2 * pair + t;
+            const int qt = qt0 + t;
             int seg = 0, row0 = 0, valid = 0;
             locate_tile<kMaxQSeg>(p.q_tile_start, p.q_len, p.n_qseg, qt, seg, row0, valid);
             const int r = (warp & 3) * 32 + lane;  // row inside the tile
@@ -777,13 +807,32 @@ cudaError_t attn_fwd_launch(const AttnParams& params, cudaStream_t stream) {
     for (int i = 0; i < kMaxKvSeg; ++i) peer_words |= p.kv_ready[i] != nullptr;
     for (int i = 0; i < kMaxQSeg; ++i) peer_words |= p.q_ready[i] != nullptr;
     if (peer_words) p.wait_limit_clk += p.peer_wait_limit_clk;
-    dim3 grid((p.n_q_tiles + 1) / 2, p.n_heads, p.batch);
-    if (p.grid_head_fastest) grid = dim3(p.n_heads, (p.n_q_tiles + 1) / 2, p.batch);
-    if (p.xchg.enabled)
-        attn_fwd_sm100_kernel<true><<<grid, kThreads, attn_fwd_smem_bytes_exchange(), stream>>>(p);
-    else
-        attn_fwd_sm100_kernel<false><<<grid, kThreads, attn_fwd_smem_bytes(), stream>>>(p);
-    return cudaPeekAtLastError();
+    p.waits_for_words = peer_words ? 1 : 0;
+    dim3 grid(p.n_heads, (p.n_q_tiles + 1) / 2, p.batch);
+    if (!p.grid_head_fastest) {
+        int dev = 0, sms = 0;
+        e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return e;
+        p.plan = cta_plan(p.n_q_tiles, p.n_heads * p.batch, sms);
+        grid = dim3(p.plan.n_ctas);
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = stream;
+    if (p.xchg.enabled) {
+        cfg.dynamicSmemBytes = attn_fwd_smem_bytes_exchange();
+        return cudaLaunchKernelEx(&cfg, attn_fwd_sm100_kernel<true>, p);
+    }
+    // May start while the kernel in front of it (the prologue) drains: the loader waits for its end.
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = peer_words ? 0 : 1;
+    cfg.dynamicSmemBytes = attn_fwd_smem_bytes();
+    return cudaLaunchKernelEx(&cfg, attn_fwd_sm100_kernel<false>, p);
 }
 
 }  // namespace f2k

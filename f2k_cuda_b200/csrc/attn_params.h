@@ -89,6 +89,43 @@ F2K_HOST_DEVICE inline int kv_walk_tile(int g, int start, int all) {
     return g >= start ? (g - start) / kTileN : tiles_a + g / kTileN;
 }
 
+// Which query tiles of which (batch, head) group a CTA takes. CTAs start in index order, one per SM, so
+// the long ones come first: first the pairs of tiles, then the single tiles - the odd last tile of every
+// group, and the pairs that were split.
+struct CtaPlan {
+    int n_pairs;    // CTAs with two tiles: pair i is pair i % pairs_per_group of group i / pairs_per_group
+    int n_split;    // the pairs n_pairs .. n_pairs + n_split - 1 are two CTAs each
+    int pairs_per_group;
+    int n_ctas;
+};
+struct CtaWork { int group, tile; bool two; };
+F2K_HOST_DEVICE inline CtaWork cta_work(const CtaPlan& c, int n_tiles, int i) {
+    CtaWork w;
+    if (i < c.n_pairs + 2 * c.n_split) {
+        const int pr = i < c.n_pairs ? i : c.n_pairs + (i - c.n_pairs) / 2;
+        w.group = pr / c.pairs_per_group;
+        w.tile  = 2 * (pr - w.group * c.pairs_per_group) + (i < c.n_pairs ? 0 : (i - c.n_pairs) & 1);
+        w.two   = i < c.n_pairs;
+    } else {
+        w.group = i - c.n_pairs - 2 * c.n_split;
+        w.tile  = n_tiles - 1;
+        w.two   = false;
+    }
+    return w;
+}
+// A CTA with one tile takes about 2/3 of the time of one with two (measured: see attn_fwd_sm100.cu).
+// The pairs that do not fill a whole wave are split when their halves, with the odd tiles, then fit
+// into one round of all SMs: the last wave takes 2/3 instead of 1.
+inline CtaPlan cta_plan(int n_tiles, int groups, int sms) {
+    CtaPlan c;
+    c.pairs_per_group = n_tiles / 2;
+    const int pairs = c.pairs_per_group * groups, odd = (n_tiles & 1) * groups, rest = pairs % sms;
+    c.n_split = 2 * rest + odd <= sms ? rest : 0;
+    c.n_pairs = pairs - c.n_split;
+    c.n_ctas  = c.n_pairs + 2 * c.n_split + odd;
+    return c;
+}
+
 struct AttnParams {
     // 4-D tensor maps, dims (fastest first): head_dim, head, token, batch;
     // box = 64 x 1 x 128 x 1 elements, 128-byte swizzle, zero fill out of bounds.
@@ -157,10 +194,12 @@ struct AttnParams {
     int           n_done;
     unsigned int  done_value;
 
-    // 0: CTAs are numbered pair-fastest (all tile pairs of a head are neighbours: the K/V of a
-    // head are shared through L2 by CTAs that run together). 1: head-fastest, so that the first
+    // 0: CTAs are numbered by `plan`, all tile pairs of a head as neighbours (the K/V of a head are
+    // shared through L2 by CTAs that run together). 1: head-fastest, so that the first
     // CTAs to run are those of the first query segments (head exchange: the local tokens).
     int grid_head_fastest;
+    CtaPlan plan;                     // set by attn_fwd_launch
+    int waits_for_words;              // set by attn_fwd_launch: some q_ready / kv_ready is not null
 
     ExchangeParams xchg;
 };

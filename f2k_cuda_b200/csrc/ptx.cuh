@@ -139,6 +139,11 @@ __device__ __forceinline__ void grid_done_publish(unsigned int* counter, unsigne
     }
 }
 
+// Programmatic dependent launch: until every kernel this launch depends on has completed and its writes
+// are visible (at once in a launch without the attribute).
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ----------------------------------------------------------------------------
 // TMA (tiled, 4-D, global -> shared, completion on an mbarrier). One destination CTA.
 // ----------------------------------------------------------------------------
