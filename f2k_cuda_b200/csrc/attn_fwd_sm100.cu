@@ -54,6 +54,7 @@
 
 #include <cuda_bf16.h>
 
+#include <cstddef>
 #include <type_traits>
 
 namespace f2k {
@@ -352,35 +353,29 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
     // Once every CTA has started, the kernel behind this one may be set up on the SMs that are free. Not
     // while this one may wait for another rank: where ranks share a GPU, that rank needs those SMs.
     if (!kWithExchange && !p.waits_for_words) grid_launch_dependents();
-    if (warp == kLoaderWarp && lane == 0) {
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(smem_u32(&ctl->q_full[i]), 1);
-            mbar_init(smem_u32(&ctl->s_full[i]), 1);
-            for (int k = 0; k < kPParts; ++k) mbar_init(smem_u32(&ctl->p_full[i][k]), 4);
-            mbar_init(smem_u32(&ctl->pv_done[i]), 1);
+    // A lane per barrier, then Q_0 and K_0 on their way, then the CTA-wide barrier: one lane that set up
+    // all barriers and issued six tiles held the other warps back for 2400 clk.
+    if (warp == kLoaderWarp) {
+        constexpr int kBars = offsetof(SmemCtl, tmem_base) / sizeof(uint64_t);
+        constexpr int kFree = offsetof(SmemCtl, s_free) / sizeof(uint64_t);
+        constexpr int kP = offsetof(SmemCtl, p_full) / sizeof(uint64_t);
+        static_assert(kBars <= 32, "a lane per barrier");
+        const bool per_warp = lane == kFree || (lane >= kP && lane < kP + 2 * kPParts);   // a softmax group's four warps arrive
+        if (lane < kBars) mbar_init(smem_u32(ctl) + lane * 8, per_warp ? 4 : 1);
+        if (lane == 0) {
+            ctl->abort = 0;
+            ctl->softmax_done = 0;
         }
-        mbar_init(smem_u32(&ctl->s_free), 4);
-        for (int i = 0; i < kStages; ++i) {
-            mbar_init(smem_u32(&ctl->kv_full[i]), 1);
-            mbar_init(smem_u32(&ctl->kv_empty[i]), 1);
-        }
-        mbar_init(smem_u32(&ctl->drain), 1);
-        if constexpr (kWithExchange)
-            for (int i = 0; i < 4; ++i) mbar_init(smem_u32(&ctl->xchg_full[0][0]) + i * 8, 1);
-        ctl->abort = 0;
-        ctl->softmax_done = 0;
         fence_mbar_init();
         fence_proxy_async_smem();
-        // Everything this kernel reads or overwrites may come from the kernel launched before it
-        // (programmatic dependent launch: this one may have started while that one drained).
-        grid_dependency_wait();
-        if (!p.waits_for_words) {
-            load_q(0);
-            for (int i = 0; i < min(kStages, 2 * n_kv); ++i) {
-                int seg, row0, valid;
-                locate_tile<kMaxKvSeg>(p.kv_tile_start, p.kv_len, p.n_kvseg, i >> 1, seg, row0, valid);
-                load_kv(seg, row0, i & 1);
-                if (i == 0 && has_t1) load_q(1);
+        __syncwarp();
+        if (lane == 0) {
+            // Everything this kernel reads or overwrites may come from the kernel launched before it
+            // (programmatic dependent launch: this one may have started while that one drained).
+            grid_dependency_wait();
+            if (!p.waits_for_words && n_kv > 0) {
+                load_q(0);
+                load_kv(0, 0, 0);
             }
         }
     }
@@ -720,12 +715,13 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
             // packets into 256-byte ones.
             const uint32_t park = smem + kSmemQ + t * kTileBytes;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                uint32_t o[32];
-                tmem_ld_x32(tO + q * 32, o);  // every lane takes part, valid row or not
+            for (int q = 0; q < 4; q += 2) {
+                uint32_t o[64];
+                tmem_ld_x32(tO + q * 32, *reinterpret_cast<uint32_t(*)[32]>(&o[0]));   // every lane takes part, valid row or not
+                tmem_ld_x32(tO + q * 32 + 32, *reinterpret_cast<uint32_t(*)[32]>(&o[32]));
                 tmem_wait_ld();
 #pragma unroll
-                for (int i = 0; i < 32; i += 8) {
+                for (int i = 0; i < 64; i += 8) {
                     uint4 v;
                     v.x = pack_bf16x2(__uint_as_float(o[i + 0]) * inv, __uint_as_float(o[i + 1]) * inv);
                     v.y = pack_bf16x2(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
@@ -736,15 +732,22 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
                 }
             }
             __syncwarp();
-            __nv_bfloat16* obase = static_cast<__nv_bfloat16*>(p.o_ptr[seg]) +
-                                   (long long)bidx * p.o_batch_stride[seg] + (long long)head * kHeadDim;
-            const int c = lane & 15;
-#pragma unroll 2
-            for (int it = 0; it < 16; ++it) {
-                const int row = (warp & 3) * 32 + it * 2 + (lane >> 4);
-                const uint4 v = ld_shared_v4(park + row * 256 + ((c ^ (row & 15)) << 4));
-                if (row < valid)
-                    *reinterpret_cast<uint4*>(obase + (long long)(row0 + row) * p.o_tok_stride[seg] + c * 8) = v;
+            const int c = lane & 15, half = lane >> 4;
+            const long long row_stride = p.o_tok_stride[seg];
+            const int first = (warp & 3) * 32 + half;
+            __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.o_ptr[seg]) + (long long)bidx * p.o_batch_stride[seg] +
+                                 (long long)head * kHeadDim + (long long)(row0 + first) * row_stride + c * 8;
+#pragma unroll
+            for (int it = 0; it < 16; it += 8) {       // eight rows read back, then written
+                uint4 v[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const int row = first + (it + k) * 2;
+                    v[k] = ld_shared_v4(park + row * 256 + ((c ^ (row & 15)) << 4));
+                }
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    if (first + (it + k) * 2 < valid) *reinterpret_cast<uint4*>(out + (it + k) * 2 * row_stride) = v[k];
             }
         }
     }
