@@ -658,8 +658,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
                 }
             }
 
-            // P = 2^(c s - c m_ref), rounded to bf16 into the first 64 columns of S_t (two keys
-            // per column); the row sum keeps the unrounded values.
+            // P = 2^(c s - c m_ref), rounded to bf16 into the 64 columns of P_t (two keys per column);
+            // the row sum keeps the unrounded values.
             const float neg_mc = -m_ref * c;
             float sum[4] = {0.f, 0.f, 0.f, 0.f};
             // A part of P is announced half a chunk after its last store was issued: by then the
@@ -708,7 +708,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
             const int r = (warp & 3) * 32 + lane;  // row inside the tile
             const float inv = 1.0f / (l_sum + 1e-30f);
             // The rows go out through the shared memory of this tile's Q (no MMA reads it any more:
-            // o_full was committed after the last of them). Each thread parks its row there, 16-byte
+            // the last pv_done comes after all of them). Each thread parks its row there, 16-byte
             // chunk c of row r at chunk position c ^ (r & 15), and the warp then writes its 32 rows
             // two at a time, 16 lanes on the 256 contiguous bytes of one row. To local memory this
             // saves partial-sector writes; to a peer's memory (head exchange) it turns 16-byte

@@ -8,10 +8,9 @@
 // 2^x comes from two places: the special-function unit (ex2.approx, 4 lanes per clock per
 // scheduler; the two softmax groups of a CTA share it) and a cubic polynomial on the FMA pipe for
 // `kPolyOf8` of every 8 key pairs. Both agree to better than 1e-4 relative, far inside the bf16
-// rounding P goes through next. Measured on the 4608-token shape, the polynomial share does not
-// pay: 1 of 8 pairs came out between 1.3 % faster and 7 % slower than none depending on how the
-// rest of the kernel happened to be scheduled, 2 of 8 and more always slower (the polynomial
-// costs issue slots the row needs elsewhere). It ships switched off (F2K_OPT_POLY_OF8 = 0).
+// rounding P goes through next. Measured with the attention kernel alone at 4608 tokens x 32 heads,
+// the polynomial share does not pay (0, 1, 2 of 8 pairs: 266, 268, 270 us; at 2125 tokens 68, 68, 72:
+// it costs issue slots the row needs elsewhere). It ships switched off (F2K_OPT_POLY_OF8 = 0).
 #pragma once
 
 #include "ptx.cuh"
