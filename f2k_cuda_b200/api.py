@@ -96,22 +96,23 @@ class _Module:
         views."""
         if not self.ok():
             return False
-        st = _lib.AttnStrides()
-        for name, t in (("q_txt", Q_txt), ("k_txt", K_txt), ("v_txt", V_txt), ("o_txt", O_txt),
-                        ("q_img", Q_img), ("k_img", K_img), ("v_img", V_img), ("o_img", O_img)):
+        token_strides = []
+        for t in (Q_txt, K_txt, V_txt, O_txt, Q_img, K_img, V_img, O_img):     # the order of AttnStrides
             if t is None:
+                token_strides.append(0)
                 continue
-            if t.dtype != torch.bfloat16 or t.dim() != 4 or t.stride(3) != 1 or t.stride(2) != t.shape[3] \
-                    or (t.shape[0] > 1 and t.stride(0) != t.shape[1] * t.stride(1)):
+            stride, shape = t.stride(), t.shape
+            if t.dtype is not _BF16 or len(shape) != 4 or stride[3] != 1 or stride[2] != shape[3] \
+                    or (shape[0] > 1 and stride[0] != shape[1] * stride[1]):
                 raise TypeError("tensors must be bfloat16 [batch, seq, heads, 128] views with dense heads and "
                                 "consecutive token rows")
-            setattr(st, name, t.stride(1))
+            token_strides.append(stride[1])
         _check_bf16(*gammas)
-        ws_bytes = 0 if workspace is None else workspace.numel() * workspace.element_size()
-        return lib.f2k_attn_forward_fused_strided(
-            self._h, _p(Q_txt), _p(K_txt), _p(V_txt), _p(Q_img), _p(K_img), _p(V_img),
-            *[_p(g) for g in gammas], *[_p(t) for t in tables], eps, _p(O_txt), _p(O_img),
-            C.byref(st), _p(workspace), ws_bytes, _stream(stream)) == _lib.F2K_OK
+        ws_bytes = 0 if workspace is None else workspace.nbytes
+        ptr = [None if t is None else t.data_ptr() for t in (Q_txt, K_txt, V_txt, Q_img, K_img, V_img, *gammas, *tables)]
+        return lib.f2k_attn_forward_fused_strided(self._h, *ptr, eps, _p(O_txt), _p(O_img),
+                                                  C.byref(_lib.AttnStrides(*token_strides)), _p(workspace), ws_bytes,
+                                                  _stream(stream)) == _lib.F2K_OK
 
     def forward_fused_host(self, hQ_txt, hK_txt, hV_txt, hQ_img, hK_img, hV_img, gammas, tables,
                            eps, hO_txt, hO_img, stream=None) -> bool:
