@@ -48,6 +48,7 @@
 // own copies and MMAs, frees its tensor memory and returns.
 
 #include "attn_launch.h"
+#include "barrier_look.h"
 #include "ptx.cuh"
 #include "row_math.cuh"
 #include "softmax_row.cuh"
@@ -123,6 +124,17 @@ __device__ __forceinline__ void locate_tile(const int* tile_start, const int* le
     row0  = (tile - tile_start[seg]) * kTileN;
     valid = min(kTileN, len[seg] - row0);
 }
+
+// The MMA warp's side of barrier_look.h.
+struct WarpBarriers {
+    volatile uint32_t* abort_flag;
+    long long limit;
+    __device__ __forceinline__ bool test(uint32_t bar_a, uint32_t par_a, uint32_t bar_b, uint32_t par_b) const {
+        return bar_a == bar_b ? mbar_test(bar_a, par_a) : mbar_test2(bar_a, par_a, bar_b, par_b);
+    }
+    __device__ __forceinline__ bool all(bool pred) const { return __all_sync(0xffffffffu, pred) != 0; }
+    __device__ __forceinline__ bool wait(uint32_t bar, uint32_t par) const { return all(mbar_wait(bar, par, abort_flag, limit)); }
+};
 
 // The MMA-issuing warp shares its scheduler with two softmax warps, so every instruction it needs per
 // MMA delays the tensor pipe. A block of MMAs is therefore one asm statement with one elected lane, and
@@ -472,20 +484,11 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
                 auto slot_off16 = [&](int n) { return (uint32_t)(n % kStages) * (kTileBytes >> 4); };
                 // A barrier that is already complete still costs the round trip of a try_wait, some
                 // 110 clk. Each wait is therefore looked at ahead (`peek`, before the MMAs in front of
-                // it are issued) and only waited for when the look found it incomplete. Two barriers
-                // are looked at in one instruction, half of the lanes each.
-                auto wait_uniform = [&](uint32_t bar, uint32_t parity) {
-                    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, wait_limit)) != 0;
-                };
-                struct Look { uint32_t bar_a, par_a, bar_b, par_b; bool seen; };
-                auto peek2 = [&](uint32_t bar_a, uint32_t par_a, uint32_t bar_b, uint32_t par_b) {
-                    return Look{bar_a, par_a, bar_b, par_b, mbar_test(lane < 16 ? bar_a : bar_b, lane < 16 ? par_a : par_b)};
-                };
-                auto peek = [&](uint32_t bar, uint32_t par) { return Look{bar, par, bar, par, mbar_test(bar, par)}; };
-                auto finish = [&](const Look& l) {
-                    if (__all_sync(0xffffffffu, l.seen)) return true;
-                    return wait_uniform(l.bar_a, l.par_a) && (l.bar_b == l.bar_a || wait_uniform(l.bar_b, l.par_b));
-                };
+                // it are issued) and only waited for when the look found it incomplete.
+                const WarpBarriers bars{abort_flag, wait_limit};
+                auto wait_uniform = [&](uint32_t bar, uint32_t par) { return bars.wait(bar, par); };
+                auto peek = [&](auto... bar_and_parity) { return look_at(bars, bar_and_parity...); };
+                auto finish = [&](const Look& l) { return f2k::finish(bars, l); };
                 auto bar_full = [&](int n) { return bar_full0 + (n % kStages) * 8; };
                 auto par_full = [&](int n) { return (uint32_t)(n / kStages) & 1u; };
                 auto release = [&](int n) { umma_commit(bar_empty0 + (n % kStages) * 8); };
@@ -541,7 +544,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
                     release(2 * j);
                     auto look_next_s0 = [&] {
                         if (j + 1 < n_kv)
-                            look_s = peek2(bar_full(2 * j + 2), par_full(2 * j + 2), bar_free, has_t1 ? 1u : (uint32_t)(j & 1));
+                            look_s = peek(bar_full(2 * j + 2), par_full(2 * j + 2), bar_free, has_t1 ? 1u : (uint32_t)(j & 1));
                     };
                     if (has_t1 && j > 0) {
                         if (!(ok = issue_pv(1, j - 1, look_p, look_next_s0))) break;
@@ -552,7 +555,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
                     if (j + 1 < n_kv) {
                         if (!(ok = finish(look_s))) break;                       // K_{j+1}; S1_j is in registers
                     }
-                    look_p = peek2(bar_full(2 * j + 1), par_full(2 * j + 1), bar_p(0, 0), j & 1);
+                    look_p = peek(bar_full(2 * j + 1), par_full(2 * j + 1), bar_p(0, 0), j & 1);
                     if (j + 1 < n_kv) issue_s(0, j + 1);
                     if (!(ok = issue_pv(0, j, look_p, [&] { if (has_t1) look_s = peek(bar_free, 0); }))) break;
                     if (!has_t1) release(2 * j + 1);

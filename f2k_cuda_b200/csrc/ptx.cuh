@@ -63,6 +63,23 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 
+// One look at two barriers, both round trips in flight together: are both phases complete?
+__device__ __forceinline__ bool mbar_test2(uint32_t bar_a, uint32_t parity_a, uint32_t bar_b, uint32_t parity_b) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred P, Q;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 Q, [%3], %4;\n\t"
+        "and.pred P, P, Q;\n\t"
+        "selp.u32 %0, 1, 0, P;\n\t"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar_a), "r"(parity_a), "r"(bar_b), "r"(parity_b)
+        : "memory");
+    return ok != 0;
+}
+
 // Bounded wait. `abort_flag` is a CTA-shared word any role sets when it gives up;
 // it is polled so that one expired wait releases every other waiter quickly.
 // Returns false when the limit ran out or the CTA is aborting. The limit is kept on the
