@@ -15,6 +15,11 @@
 //
 // All of them are HBM-bound: 16-byte loads/stores, a half-warp (dim 128) or a warp per
 // 128-element head row, grid sized as a multiple of the SM count, grid-stride loop.
+//
+// The head_dim 128 kernels may start while the kernel in front of them still runs and writes what they
+// read, whatever it is: rows, gains, tables or positions. So they read with plain loads only, behind
+// griddepcontrol.wait: __ldg and `const __restrict__` promise that nobody writes the data for as long as the
+// kernel lives, and plain `__restrict__` that the wait does not touch it; either lets a load move ahead of it.
 
 #include "attn_launch.h"
 #include "row_math.cuh"
@@ -67,16 +72,15 @@ qk_prologue_kernel(const __grid_constant__ QkPrologueParams p) {
         const unsigned trow = lr / (unsigned)p.n_heads;         // token row over batch * seq
         const unsigned tok = trow % (unsigned)job.seq;
         const unsigned hd0 = lr - trow * (unsigned)p.n_heads;   // first head of the group
-        // plain loads of x: y may alias x, so x is not read-only for the kernel's lifetime. A token
-        // row of x may be a slice of a wider row (x_tok_stride); y is always dense.
+        // A token row of x may be a slice of a wider row (x_tok_stride); y is always dense.
         const uint4* src = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(job.x) +
                                                           (long long)trow * job.x_tok_stride + hd0 * kHeadDim);
         uint4 raw[kGroup];
 #pragma unroll
         for (int u = 0; u < kGroup; ++u) raw[u] = src[u * 16 + hl];
-        const uint4  graw = __ldg(reinterpret_cast<const uint4*>(job.gamma) + hl);
-        const float4 c4 = __ldg(reinterpret_cast<const float4*>(job.cos_tab + (long long)tok * 64) + hl);
-        const float4 s4 = __ldg(reinterpret_cast<const float4*>(job.sin_tab + (long long)tok * 64) + hl);
+        const uint4  graw = reinterpret_cast<const uint4*>(job.gamma)[hl];
+        const float4 c4 = reinterpret_cast<const float4*>(job.cos_tab + (long long)tok * 64)[hl];
+        const float4 s4 = reinterpret_cast<const float4*>(job.sin_tab + (long long)tok * 64)[hl];
         float g[8];
         unpack8(graw, g);
         const float cs[4] = {c4.x, c4.y, c4.z, c4.w};
@@ -170,13 +174,13 @@ qkv_scatter_kernel(const __grid_constant__ QkvScatterParams p) {
 constexpr int kRowsAhead = 4;
 
 __global__ void __launch_bounds__(kBlock)
-rmsnorm_rows128_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ gamma,
+rmsnorm_rows128_kernel(const __nv_bfloat16* x, const __nv_bfloat16* gamma,
                        __nv_bfloat16* y, long long rows, float eps) {  // y may alias x
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int hl = threadIdx.x & 15;
     const long long n_hw = (long long)gridDim.x * (kBlock / 16);
-    const uint4 graw = __ldg(reinterpret_cast<const uint4*>(gamma) + hl);
+    const uint4 graw = reinterpret_cast<const uint4*>(gamma)[hl];
     float g[8];
     unpack8(graw, g);
     for (long long row0 = ((long long)blockIdx.x * (kBlock / 16) + (threadIdx.x >> 4)) * kRowsAhead; row0 < rows;
@@ -239,8 +243,8 @@ rmsnorm_rows_generic_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restr
 // x'[2k] = x[2k] c - x[2k+1] s ; x'[2k+1] = x[2k] s + x[2k+1] c with c, s = table[pos][k].
 // ---------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kBlock)
-rope4_rows128_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ cos_tab,
-                     const float* __restrict__ sin_tab, const int32_t* __restrict__ pos_ids,
+rope4_rows128_kernel(__nv_bfloat16* x, const float* cos_tab,
+                     const float* sin_tab, const int32_t* pos_ids,
                      long long rows, int seq_max) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -254,7 +258,7 @@ rope4_rows128_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ co
         for (int u = 0; u < kRowsAhead; ++u)
             if (row0 + u < rows) {
                 raw[u] = reinterpret_cast<const uint4*>(x + (row0 + u) * 128)[hl];
-                const int pid = __ldg(pos_ids + row0 + u);
+                const int pid = pos_ids[row0 + u];
                 pos[u] = pid >= seq_max ? seq_max - 1 : (pid < 0 ? 0 : pid);
             }
         float4 c4, s4;
@@ -262,8 +266,8 @@ rope4_rows128_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ co
         for (int u = 0; u < kRowsAhead; ++u) {
             if (row0 + u >= rows) break;
             if (u == 0 || pos[u] != pos[u - 1]) {            // the heads of one token share a table row
-                c4 = __ldg(reinterpret_cast<const float4*>(cos_tab + (long long)pos[u] * 64) + hl);
-                s4 = __ldg(reinterpret_cast<const float4*>(sin_tab + (long long)pos[u] * 64) + hl);
+                c4 = reinterpret_cast<const float4*>(cos_tab + (long long)pos[u] * 64)[hl];
+                s4 = reinterpret_cast<const float4*>(sin_tab + (long long)pos[u] * 64)[hl];
             }
             float v[8], o[8];
             unpack8(raw[u], v);
