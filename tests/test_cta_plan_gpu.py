@@ -37,6 +37,28 @@ def test_rows_do_not_depend_on_the_plan(S):
         assert_parity(host_f32(part[0, :, n]), (torch.softmax(s, -1) @ v[0, :, h].float()).cpu().numpy(), f"head {h}")
 
 
+# The lazy reference maximum moves (and O is rescaled in tensor memory) when a tile's maximum exceeds it by 8 in
+# log2 units, 5.5 nats: score levels per key tile that rise by 8 nats and more from tile to tile in every second
+# head, and lie anywhere from 0 to 40 in the others. Values within 4.7 (400 thousand N(0, 1)): 2^-9 of that for the rounding of P
+# and as much for the output's stay below the gate.
+@pytest.mark.parametrize("S", [256, 300, 400, 1100])
+def test_moving_maximum_in_both_kinds_of_cta(S):
+    import torch
+    H, tiles = 160, -(-S // 128)
+    q, k, v = [dev_bf16(normal_bits(0x3A71 + i, S, (1, S, H, 128))) for i in range(3)]
+    level = np.random.default_rng(S).uniform(0, 40, (H, tiles))
+    level[1::2] = 12 * np.arange(tiles) + level[1::2] / 10
+    q[..., 0] = 128 ** 0.5
+    k[..., 0] = torch.from_numpy(level.T.repeat(128, axis=0)[:S].astype(np.float32)).cuda()
+    whole = _forward(q, k, v)
+    few = [0, 77, 159]
+    part = _forward(*[x[:, :, few].contiguous() for x in (q, k, v)])
+    assert torch.equal(whole[:, :, few], part)
+    for n, h in enumerate(few):
+        s = (q[0, :, h].double() @ k[0, :, h].double().T) * 128 ** -0.5
+        assert_parity(host_f32(part[0, :, n]), (torch.softmax(s, -1) @ v[0, :, h].double()).cpu().numpy(), f"head {h}")
+
+
 @pytest.mark.parametrize("rows", [1, 2, 3, 4, 5, 63, 64, 65, 148 * 8 * 64 + 3])
 def test_row_kernels_at_the_edges_of_their_groups(rows):
     """Every row alone gives the same bits as the row inside a call (a half-warp takes four at a time), and
