@@ -14,6 +14,9 @@ PROGRAM = r"""
 #include <vector>
 using namespace f2k;
 int main() {
+    const CtaPlan ragged = cta_plan(17, 24, 148), ordinary = cta_plan(9, 32, 148);
+    if (ragged.n_pairs != 148 || ragged.n_split != 44 || ragged.n_ctas != 148 + 2 * 44 + 24 ||
+        ordinary.n_pairs != 128 || ordinary.n_split != 0 || ordinary.n_ctas != 128 + 32) { std::printf("known plans\n"); return 1; }
     for (int sms : {1, 7, 148})
         for (int tiles = 1; tiles <= 140; tiles += (tiles < 40 ? 1 : 7))
             for (int groups : {1, 2, 3, 4, 12, 24, 31, 32, 64, 128}) {
@@ -33,6 +36,8 @@ int main() {
                 }
                 for (int n : seen)
                     if (n != 1) { std::printf("sms %d tiles %d groups %d: a tile %d times\n", sms, tiles, groups, n); return 1; }
+                const int rest = tiles / 2 * groups % sms, odd = tiles % 2 * groups;
+                if (c.n_split != (2 * rest + odd <= sms ? rest : 0)) { std::printf("split rule\n"); return 1; }
                 if (c.n_split > 0 && (c.n_pairs % sms != 0 || c.n_ctas - c.n_pairs > sms)) { std::printf("split\n"); return 1; }
             }
     return 0;
