@@ -59,9 +59,10 @@ def test_moving_maximum_in_both_kinds_of_cta(S):
         assert_parity(host_f32(part[0, :, n]), (torch.softmax(s, -1) @ v[0, :, h].double()).cpu().numpy(), f"head {h}")
 
 
-@pytest.mark.parametrize("rows", [1, 2, 3, 4, 5, 63, 64, 65, 148 * 8 * 64 + 3])
+@pytest.mark.parametrize("rows", [1, 2, 3, 4, 5, 63, 64, 65, 148 * 8 * 64 + 3]
+                         + [148 * 8 * 16 + n for n in (0, 1, 2, 3, 4)])       # one row at a time up to here, then four
 def test_row_kernels_at_the_edges_of_their_groups(rows):
-    """Every row alone gives the same bits as the row inside a call (a half-warp takes four at a time), and
+    """Every row alone gives the same bits as the row inside a call (a half-warp takes one or four at a time), and
     nothing behind the last row is written."""
     import torch
 
