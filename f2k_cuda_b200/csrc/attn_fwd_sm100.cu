@@ -73,18 +73,14 @@ constexpr uint32_t kBoxBytes  = kTileBytes / 2;         // one 128 x 64 TMA box
 constexpr uint32_t kTmemCols  = 512;
 constexpr uint32_t kColS = 0, kColP0 = 128, kColP1 = 192, kColO0 = 256, kColO1 = 384;
 constexpr float kLazyThreshold = 8.0f;  // log2 units
+constexpr int kPParts = 2;     // P is handed to the MMA warp in halves (1, 2, 4 parts: 269, 266, 269 us at 4608 tokens x 32 heads)
+constexpr int kPvSteps = 4;    // k-steps of 16 keys per part: umma_ts_x4
+static_assert(kPParts * kPvSteps * 16 == kTileN, "the parts cover the key tile");
 
 // Tuning switches (compile-time; the defaults are what ships).
 #ifndef F2K_OPT_SETMAXNREG
 #define F2K_OPT_SETMAXNREG 1   // softmax warpgroups take registers from the load/MMA warpgroup
 #endif
-#ifndef F2K_OPT_P_PARTS
-#define F2K_OPT_P_PARTS 2      // P is handed to the MMA warp in this many parts (1, 2 or 4; 269, 266, 269 us at 4608 tokens x 32 heads)
-#endif
-#ifndef F2K_OPT_POLY_OF8
-#define F2K_OPT_POLY_OF8 0     // of every 8 key pairs, how many take 2^x on the FMA pipe (0..8); see softmax_row.cuh
-#endif
-constexpr int kPParts = F2K_OPT_P_PARTS;
 #ifndef F2K_OPT_REGS_SOFTMAX
 #define F2K_OPT_REGS_SOFTMAX 208
 #endif
@@ -156,8 +152,8 @@ __device__ __forceinline__ void issue_qk(uint32_t d_tmem, uint64_t q_desc, uint6
 template <int kPart>
 __device__ __forceinline__ void issue_pv_part(uint32_t d_tmem, uint32_t p_tmem, uint64_t v_desc, uint32_t accumulate) {
     constexpr uint32_t idesc = umma_idesc_bf16(kTileM, kHeadDim, /*b_mn_major=*/true);
-    constexpr int kSteps = 8 / kPParts, kk = kPart * kSteps;
-    umma_ts_xn<kSteps>(d_tmem, p_tmem + kk * 8, v_desc + kk * (2048 >> 4), idesc, kPart > 0 ? 1u : accumulate);
+    constexpr int kk = kPart * kPvSteps;
+    umma_ts_x4(d_tmem, p_tmem + kk * 8, v_desc + kk * (2048 >> 4), idesc, kPart > 0 ? 1u : accumulate);
 }
 
 // Head exchange by one of the CTA's two spare warps (see ExchangeParams). A chunk is 16 tokens of
@@ -672,7 +668,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 uint32_t pk[16];
-                exp_chunk16<F2K_OPT_POLY_OF8>(&s[q * 32], pk, c, neg_mc, sum);
+                exp_chunk16(&s[q * 32], pk, c, neg_mc, sum);
                 if (pending >= 0) {
                     tmem_wait_st();
                     tc_fence_before_sync();
@@ -680,7 +676,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
                     if (lane == 0) mbar_arrive(smem_u32(&ctl->p_full[t][0]) + pending * 8);
                     pending = -1;
                 }
-                exp_chunk16<F2K_OPT_POLY_OF8>(&s[q * 32 + 16], pk + 8, c, neg_mc, sum);
+                exp_chunk16(&s[q * 32 + 16], pk + 8, c, neg_mc, sum);
                 if (q == 0 && !__all_sync(0xffffffffu, pv_seen)) {   // P_t of the previous key tile is still being read
                     ok = mbar_wait(smem_u32(&ctl->pv_done[t]), (j - 1) & 1, abort_flag, wait_limit);
                     ok = __all_sync(0xffffffffu, ok);

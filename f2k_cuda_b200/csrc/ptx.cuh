@@ -335,41 +335,34 @@ __device__ __forceinline__ void umma_ss_x8(uint32_t d_tmem, uint64_t a_desc, uin
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc)
         : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem] over kSteps k-steps of 16: 8 columns of A and 2048 bytes of B each.
-#define F2K_UMMA_TS_STEP(K)                                  \
-    "add.s32 a, %1, " #K " * 8;\n\t"                         \
-    "add.s64 b, %2, " #K " * 128;\n\t"                       \
-    "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, more;\n\t"
-#define F2K_UMMA_TS(STEPS)                                                                   \
-    asm volatile(                                                                            \
-        "{\n\t"                                                                              \
-        ".reg .pred pe, p, more;\n\t"                                                        \
-        ".reg .b32 a;\n\t"                                                                   \
-        ".reg .b64 b;\n\t"                                                                   \
-        "elect.sync _|pe, 0xffffffff;\n\t"                                                   \
-        "setp.ne.b32 p, %4, 0;\n\t"                                                          \
-        "setp.eq.b32 more, 0, 0;\n\t"                                                        \
-        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t" STEPS            \
-        "}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory")
-template <int kSteps>
-__device__ __forceinline__ void umma_ts_xn(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+// D[tmem] (+)= A[tmem] * B[smem] over 4 k-steps of 16: 8 columns of A and 2048 bytes of B each.
+__device__ __forceinline__ void umma_ts_x4(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
                                            uint32_t accumulate) {
-    static_assert(kSteps == 2 || kSteps == 4 || kSteps == 6 || kSteps == 8, "written out below");
-    if constexpr (kSteps == 2)
-        F2K_UMMA_TS(F2K_UMMA_TS_STEP(1));
-    else if constexpr (kSteps == 4)
-        F2K_UMMA_TS(F2K_UMMA_TS_STEP(1) F2K_UMMA_TS_STEP(2) F2K_UMMA_TS_STEP(3));
-    else if constexpr (kSteps == 6)
-        F2K_UMMA_TS(F2K_UMMA_TS_STEP(1) F2K_UMMA_TS_STEP(2) F2K_UMMA_TS_STEP(3) F2K_UMMA_TS_STEP(4) F2K_UMMA_TS_STEP(5));
-    else
-        F2K_UMMA_TS(F2K_UMMA_TS_STEP(1) F2K_UMMA_TS_STEP(2) F2K_UMMA_TS_STEP(3) F2K_UMMA_TS_STEP(4) F2K_UMMA_TS_STEP(5)
-                    F2K_UMMA_TS_STEP(6) F2K_UMMA_TS_STEP(7));
+    asm volatile(
+        "{\n\t"
+        ".reg .pred pe, p, more;\n\t"
+        ".reg .b32 a;\n\t"
+        ".reg .b64 b;\n\t"
+        "elect.sync _|pe, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.eq.b32 more, 0, 0;\n\t"
+        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        "add.s32 a, %1, 8;\n\t"
+        "add.s64 b, %2, 128;\n\t"
+        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, more;\n\t"
+        "add.s32 a, %1, 16;\n\t"
+        "add.s64 b, %2, 256;\n\t"
+        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, more;\n\t"
+        "add.s32 a, %1, 24;\n\t"
+        "add.s64 b, %2, 384;\n\t"
+        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, more;\n\t"
+        "}\n"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
 }
-#undef F2K_UMMA_TS
-#undef F2K_UMMA_TS_STEP
 // Arrive (count 1) on `bar` once every tcgen05 operation the elected lane issued before the
 // commit has completed. elect.sync picks the same lane every time for a full warp, so the
-// commit tracks the MMAs issued through umma_ss_x8 / umma_ts_xn.
+// commit tracks the MMAs issued through umma_ss_x8 / umma_ts_x4.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile(
         "{\n\t"
