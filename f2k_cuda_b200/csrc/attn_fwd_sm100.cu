@@ -32,8 +32,10 @@
 // What bounds it: the issuing warp shares its scheduler with two softmax warps, and per key tile it
 // needed some 3000 clk for what the tensor pipe does in 2048: 110 clk per barrier that was complete
 // anyway, 30 per MMA. Hence the looks ahead at barriers, one asm block and one elected lane per run of
-// MMAs, and operands the compiler knows to be uniform (278 -> 266 us). What is left is the
-// special-function unit, which the two groups share (2048 clk per key tile), and the power cap.
+// MMAs, and operands the compiler knows to be uniform (278 -> 266 us). An iteration is now some 2850 clk;
+// the tensor pipe and the special-function unit, which the two groups share, are both 68 % busy (2048 clk
+// each per key tile), and the rest is hand-overs, tensor-memory latency and a CTA's start and epilogue.
+// The power cap comes on top in calls back to back for long.
 //
 // Online softmax with a lazy reference maximum: the exponent reference of a row
 // only moves when some row of the warp sees a tile maximum more than 2^8 above it;
@@ -394,8 +396,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ AttnParams p) {
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    // All 512 columns are taken, so the allocation starts at column 0: a constant, which spares every
-    // tensor-memory address a register (checked: anything else ends the CTA with the status word set).
+    // All 512 columns are taken, so the allocation can only start at column 0: a constant, which spares
+    // every tensor-memory address a register (were it anything else, the status word would say so).
     constexpr uint32_t tmem = 0;
     if (*reinterpret_cast<volatile uint32_t*>(&ctl->tmem_base) != tmem) ctl->abort = 1;
 
