@@ -83,7 +83,7 @@ class _Module:
         _check_bf16(Q_txt, K_txt, V_txt, Q_img, K_img, V_img, O_txt, O_img, *gammas)
         ws_bytes = 0 if workspace is None else workspace.nbytes
         # The smallest calls are bound by what happens here (13 to 16 us of 18 with one _p() call per tensor
-        # and a c_void_p object each, 7 to 8 of 15 now), so all addresses are taken in one go.
+        # and a c_void_p object each, 4.5 of 12 now), so all addresses are taken in one go.
         ptr = [None if t is None else t.data_ptr() for t in (Q_txt, K_txt, V_txt, Q_img, K_img, V_img, *gammas, *tables)]
         return lib.f2k_attn_forward_fused(self._h, *ptr, eps, _p(O_txt), _p(O_img), _p(workspace), ws_bytes,
                                           _stream(stream)) == _lib.F2K_OK
