@@ -6,6 +6,7 @@
 #include "f2k_attn.h"
 
 #include "attn_launch.h"
+#include "handle_device.h"
 
 #include <algorithm>
 #include <cmath>
@@ -428,6 +429,7 @@ int f2k_attn_forward(f2k_attn* h, const void* q_txt, const void* k_txt, const vo
     (void)workspace_bytes;  // nothing to check: this path needs no workspace
     if (!h) return F2K_ERR_INVALID;
     if (!h->valid) return F2K_ERR_INVALID;  // keeps the creation error as last_error
+    if (const int rc = check_current_device(h->device, h->err)) return rc;
     const int rc = prepare_params(h, q_txt, k_txt, v_txt, q_img, k_img, v_img, o_txt, o_img);
     if (rc != F2K_OK) return rc;
     const cudaError_t e = attn_fwd_launch(h->params, static_cast<cudaStream_t>(stream));
@@ -456,6 +458,7 @@ int f2k_attn_forward_fused_strided(f2k_attn* h, const void* q_txt, const void* k
                                    void* workspace, size_t workspace_bytes, void* stream) {
     if (!h) return F2K_ERR_INVALID;
     if (!h->valid) return F2K_ERR_INVALID;
+    if (const int rc = check_current_device(h->device, h->err)) return rc;
     if (workspace_bytes < h->fused_ws() || !workspace)
         return fail(h, F2K_ERR_WORKSPACE, "workspace too small");
     const f2k_attn_config& c = h->cfg;
@@ -542,6 +545,7 @@ int f2k_attn_forward_fused_host(f2k_attn* h, const void* hq_txt, const void* hk_
                                 float eps, void* ho_txt, void* ho_img, void* stream) {
     if (!h) return F2K_ERR_INVALID;
     if (!h->valid) return F2K_ERR_INVALID;
+    if (const int rc = check_current_device(h->device, h->err)) return rc;
     const f2k_attn_config& c = h->cfg;
     const bool has_txt = c.seq_txt > 0;
     if (!hq_img || !hk_img || !hv_img || !ho_img ||
@@ -669,6 +673,8 @@ int f2k_attn_forward_fused_host(f2k_attn* h, const void* hq_txt, const void* hk_
 int f2k_attn_device_status(f2k_attn* h, int* status_out) {
     if (!h || !h->valid) return F2K_ERR_INVALID;
     int st = 0;
+    const OnDevice here(h->device);
+    if (here.error != cudaSuccess) return fail_cuda(h, "cudaSetDevice", here.error);
     cudaError_t e = cudaDeviceSynchronize();
     if (e != cudaSuccess) return fail_cuda(h, "cudaDeviceSynchronize", e);
     e = cudaMemcpy(&st, h->d_status, sizeof st, cudaMemcpyDeviceToHost);

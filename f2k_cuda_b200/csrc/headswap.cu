@@ -45,6 +45,7 @@
 #include "f2k_attn.h"
 
 #include "attn_launch.h"
+#include "handle_device.h"
 
 #include <algorithm>
 #include <cmath>
@@ -77,6 +78,7 @@ struct f2k_hx {
     float  scale = 0.f;
     bool   valid = false;
     std::string err;
+    int    device = -1;
     unsigned char* buf = nullptr;
     size_t shard_bytes = 0, total_bytes = 0, flags_off = 0;
     int    hpr = 0;                          // heads per rank
@@ -178,10 +180,10 @@ int f2k_hx_create(const f2k_seqpar_config* cfg, f2k_hx** out) {
     h->total_bytes = h->flags_off + f2k_hx::kControlBytes +
                      ((size_t)2 * cfg->world * 3 * h->n_tiles * sizeof(unsigned int) + 255) / 256 * 256;
 
-    int dev = 0, major = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    int major = 0;
+    cudaError_t e = cudaGetDevice(&h->device);
     if (e != cudaSuccess) return fail_cuda(h, "cudaGetDevice", e);
-    e = cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev);
+    e = cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, h->device);
     if (e != cudaSuccess) return fail_cuda(h, "cudaDeviceGetAttribute", e);
     if (major != 10) return fail(h, F2K_ERR_UNSUPPORTED, "this library contains sm_100a code only");
     h->encode = reinterpret_cast<EncodeTiledFn>(driver_entry("cuTensorMapEncodeTiled"));
@@ -244,6 +246,7 @@ int f2k_hx_exchange_in(f2k_hx* h, const void* q_raw, const void* k_raw, const vo
                        const void* gamma_k, const float* cos_local, const float* sin_local, float eps,
                        void* stream) {
     if (!h || !h->valid) return F2K_ERR_INVALID;
+    if (const int rc = check_current_device(h->device, h->err)) return rc;
     if (!q_raw || !k_raw || !v || !gamma_q || !gamma_k || !cos_local || !sin_local)
         return fail(h, F2K_ERR_INVALID, "null tensor pointer");
     for (const void* ptr : {q_raw, k_raw, v, gamma_q, gamma_k, static_cast<const void*>(cos_local),
@@ -293,6 +296,7 @@ int f2k_hx_exchange_in_copy(f2k_hx* h, const void* q_raw, const void* k_raw, con
                             const void* gamma_k, const float* cos_local, const float* sin_local, float eps,
                             void* stream) {
     if (!h || !h->valid) return F2K_ERR_INVALID;
+    if (const int rc = check_current_device(h->device, h->err)) return rc;
     if (!q_raw || !k_raw || !v || !gamma_q || !gamma_k || !cos_local || !sin_local)
         return fail(h, F2K_ERR_INVALID, "null tensor pointer");
     for (const void* ptr : {q_raw, k_raw, v, gamma_q, gamma_k, static_cast<const void*>(cos_local),
@@ -389,6 +393,7 @@ int f2k_hx_exchange_in_copy(f2k_hx* h, const void* q_raw, const void* k_raw, con
 
 int f2k_hx_attend(f2k_hx* h, void* stream) {
     if (!h || !h->valid) return F2K_ERR_INVALID;
+    if (const int rc = check_current_device(h->device, h->err)) return rc;
     if (h->phase != f2k_hx::kExchanged) return fail(h, F2K_ERR_INVALID, "attend without exchange_in");
     const f2k_seqpar_config& c = h->cfg;
     const int set = h->epoch & 1;
@@ -493,6 +498,7 @@ void fill_exchange_order(ExchangeParams& x, int world, int seq_local, int heads_
 int f2k_hx_forward(f2k_hx* h, const void* q_raw, const void* k_raw, const void* v, const void* gamma_q,
                    const void* gamma_k, const float* cos_local, const float* sin_local, float eps, void* stream) {
     if (!h || !h->valid) return F2K_ERR_INVALID;
+    if (const int rc = check_current_device(h->device, h->err)) return rc;
     if (!q_raw || !k_raw || !v || !gamma_q || !gamma_k || !cos_local || !sin_local)
         return fail(h, F2K_ERR_INVALID, "null tensor pointer");
     for (const void* ptr : {q_raw, k_raw, v, gamma_q, gamma_k, static_cast<const void*>(cos_local),
@@ -634,6 +640,7 @@ int f2k_hx_kv_walk_tile(int world, int seq_local, int dst_rank, int token, int* 
 
 int f2k_hx_output(f2k_hx* h, void** o_local, void* stream) {
     if (!h || !h->valid) return F2K_ERR_INVALID;
+    if (const int rc = check_current_device(h->device, h->err)) return rc;
     if (h->phase != f2k_hx::kAttended) return fail(h, F2K_ERR_INVALID, "output without attend");
     const int set = h->epoch & 1;
     for (int s = 0; s < h->cfg.world; ++s)
@@ -648,6 +655,8 @@ int f2k_hx_output(f2k_hx* h, void** o_local, void* stream) {
 int f2k_hx_device_status(f2k_hx* h, int* status_out) {
     if (!h || !h->valid) return F2K_ERR_INVALID;
     int st = 0;
+    const OnDevice here(h->device);
+    if (here.error != cudaSuccess) return fail_cuda(h, "cudaSetDevice", here.error);
     cudaError_t e = cudaDeviceSynchronize();
     if (e != cudaSuccess) return fail_cuda(h, "cudaDeviceSynchronize", e);
     e = cudaMemcpy(&st, h->d_status, sizeof st, cudaMemcpyDeviceToHost);

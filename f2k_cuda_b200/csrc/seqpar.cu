@@ -38,6 +38,7 @@
 #include "f2k_attn.h"
 
 #include "attn_launch.h"
+#include "handle_device.h"
 
 #include <cmath>
 #include <cstdio>
@@ -72,6 +73,7 @@ struct f2k_seqpar {
     float  scale = 0.f;
     bool   valid = false;
     std::string err;
+    int    device = -1;
     unsigned char* buf = nullptr;       // the allocation described above
     size_t shard_bytes = 0, set_bytes = 0, total_bytes = 0, flags_off = 0;
     using WaitValue32Fn = CUresult (*)(CUstream, CUdeviceptr, cuuint32_t, unsigned int);
@@ -158,10 +160,10 @@ int f2k_seqpar_create(const f2k_seqpar_config* cfg, f2k_seqpar** out) {
     h->total_bytes = h->flags_off +
                      align_up(((size_t)2 * cfg->world * (f2k_seqpar::kMaxGroups + 1) + 1) * sizeof(unsigned int), kAlign);
 
-    int dev = 0, major = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    int major = 0;
+    cudaError_t e = cudaGetDevice(&h->device);
     if (e != cudaSuccess) return fail_cuda(h, "cudaGetDevice", e);
-    e = cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev);
+    e = cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, h->device);
     if (e != cudaSuccess) return fail_cuda(h, "cudaDeviceGetAttribute", e);
     if (major != 10) return fail(h, F2K_ERR_UNSUPPORTED, "this library contains sm_100a code only");
     h->encode  = reinterpret_cast<EncodeTiledFn>(driver_fn("cuTensorMapEncodeTiled"));
@@ -230,6 +232,7 @@ int f2k_seqpar_local_kv(f2k_seqpar* h, void** k, void** v) {
 int f2k_seqpar_forward(f2k_seqpar* h, const void* q_local, void* o_local, int overlap,
                        void* compute_stream, void* copy_stream) {
     if (!h || !h->valid) return F2K_ERR_INVALID;
+    if (const int rc = check_current_device(h->device, h->err)) return rc;
     if (!q_local || !o_local) return fail(h, F2K_ERR_INVALID, "null tensor pointer");
     if ((reinterpret_cast<uintptr_t>(q_local) & 15u) || (reinterpret_cast<uintptr_t>(o_local) & 15u))
         return fail(h, F2K_ERR_INVALID, "q_local and o_local must be 16-byte aligned");
@@ -382,6 +385,8 @@ int f2k_seqpar_forward(f2k_seqpar* h, const void* q_local, void* o_local, int ov
 int f2k_seqpar_device_status(f2k_seqpar* h, int* status_out) {
     if (!h || !h->valid) return F2K_ERR_INVALID;
     int st = 0;
+    const OnDevice here(h->device);
+    if (here.error != cudaSuccess) return fail_cuda(h, "cudaSetDevice", here.error);
     cudaError_t e = cudaDeviceSynchronize();
     if (e != cudaSuccess) return fail_cuda(h, "cudaDeviceSynchronize", e);
     e = cudaMemcpy(&st, h->d_status, sizeof st, cudaMemcpyDeviceToHost);

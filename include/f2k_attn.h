@@ -21,6 +21,9 @@
  *    which are 16-byte aligned.)
  *  - A handle holds mutable state (error text, cached TMA descriptors): use it from
  *    one host thread at a time. Distinct handles on distinct streams are independent.
+ *  - A handle belongs to the device that is current when it is created. A call that would launch or
+ *    queue something for it while another device is current is refused with F2K_ERR_INVALID; the
+ *    *_device_status functions synchronise the handle's device, whichever one is current.
  *  - There is no CPU fallback and no other GPU path: on a device that is not
  *    compute capability 10.x, or for head_dim != 128, creation fails with a message.
  *  - Three environment variables override choices the library otherwise makes itself; they
