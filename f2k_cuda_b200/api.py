@@ -17,17 +17,12 @@ import torch
 
 from . import _lib
 from ._lib import AttnConfig, lib
+from ._stream import stream_handle
 
 
 def _p(t):
     """Device (or host) address of a tensor, None -> NULL."""
     return None if t is None else t.data_ptr()      # an int: ctypes converts it faster than a c_void_p object
-
-
-def _stream(stream):
-    if stream is None:      # the current stream's handle without a Stream object around it: 192 tokens x 4 heads 15.5 -> 12.0 us
-        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
-    return stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream)
 
 
 _BF16 = torch.bfloat16
@@ -86,7 +81,7 @@ class _Module:
         # and a c_void_p object each, 4.5 of 12 now), so all addresses are taken in one go.
         ptr = [None if t is None else t.data_ptr() for t in (Q_txt, K_txt, V_txt, Q_img, K_img, V_img, *gammas, *tables)]
         return lib.f2k_attn_forward_fused(self._h, *ptr, eps, _p(O_txt), _p(O_img), _p(workspace), ws_bytes,
-                                          _stream(stream)) == _lib.F2K_OK
+                                          stream_handle(stream)) == _lib.F2K_OK
 
     def forward_fused_strided(self, Q_txt, K_txt, V_txt, Q_img, K_img, V_img, gammas, tables, eps,
                               O_txt, O_img, workspace, stream=None) -> bool:
@@ -112,7 +107,7 @@ class _Module:
         ptr = [None if t is None else t.data_ptr() for t in (Q_txt, K_txt, V_txt, Q_img, K_img, V_img, *gammas, *tables)]
         return lib.f2k_attn_forward_fused_strided(self._h, *ptr, eps, _p(O_txt), _p(O_img),
                                                   C.byref(_lib.AttnStrides(*token_strides)), _p(workspace), ws_bytes,
-                                                  _stream(stream)) == _lib.F2K_OK
+                                                  stream_handle(stream)) == _lib.F2K_OK
 
     def forward_fused_host(self, hQ_txt, hK_txt, hV_txt, hQ_img, hK_img, hV_img, gammas, tables,
                            eps, hO_txt, hO_img, stream=None) -> bool:
@@ -123,7 +118,7 @@ class _Module:
         return lib.f2k_attn_forward_fused_host(
             self._h, _p(hQ_txt), _p(hK_txt), _p(hV_txt), _p(hQ_img), _p(hK_img), _p(hV_img),
             *[_p(g) for g in gammas], *[_p(t) for t in tables], eps, _p(hO_txt), _p(hO_img),
-            _stream(stream)) == _lib.F2K_OK
+            stream_handle(stream)) == _lib.F2K_OK
 
 
 class Attention(_Module):
@@ -145,7 +140,7 @@ class Attention(_Module):
             return False
         _check_bf16(Q, K, V, O)
         return lib.f2k_attn_forward(self._h, None, None, None, _p(Q), _p(K), _p(V), None, _p(O),
-                                    None, 0, _stream(stream)) == _lib.F2K_OK
+                                    None, 0, stream_handle(stream)) == _lib.F2K_OK
 
     def forward_fused_single(self, Q, K, V, gamma_q, gamma_k, cos, sin, eps, O, workspace, stream=None,
                              strided: bool = False) -> bool:
@@ -184,19 +179,19 @@ class JointAttention(_Module):
         _check_bf16(Q_txt, K_txt, V_txt, Q_img, K_img, V_img, O_txt, O_img)
         return lib.f2k_attn_forward(self._h, _p(Q_txt), _p(K_txt), _p(V_txt), _p(Q_img), _p(K_img),
                                     _p(V_img), _p(O_txt), _p(O_img), _p(workspace), workspace_size,
-                                    _stream(stream)) == _lib.F2K_OK
+                                    stream_handle(stream)) == _lib.F2K_OK
 
 
 def rmsnorm_bf16(x, gamma, y, batch_rows: int, dim: int, eps: float, stream=None) -> bool:
     """Mirror of f2k::cuda::rmsnorm_bf16 (y may be x)."""
-    return lib.f2k_rmsnorm_bf16(_p(x), _p(gamma), _p(y), batch_rows, dim, eps, _stream(stream)) == _lib.F2K_OK
+    return lib.f2k_rmsnorm_bf16(_p(x), _p(gamma), _p(y), batch_rows, dim, eps, stream_handle(stream)) == _lib.F2K_OK
 
 
 def rope_4axis_inplace_bf16(x, cos_table, sin_table, pos_ids, batch_rows: int, head_dim: int,
                             seq_max: int, stream=None) -> bool:
     """Mirror of f2k::cuda::rope_4axis_inplace_bf16."""
     return lib.f2k_rope_4axis_inplace_bf16(_p(x), _p(cos_table), _p(sin_table), _p(pos_ids),
-                                           batch_rows, head_dim, seq_max, _stream(stream)) == _lib.F2K_OK
+                                           batch_rows, head_dim, seq_max, stream_handle(stream)) == _lib.F2K_OK
 
 
 def build_rope_4axis_tables(axes_dim, token_positions, theta: float):

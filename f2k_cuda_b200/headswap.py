@@ -11,6 +11,7 @@ import ctypes as C
 
 from . import _lib
 from ._lib import SeqParConfig, lib
+from ._stream import stream_handle
 from .seqpar import _tensor_from_ptr
 
 
@@ -95,17 +96,12 @@ class HeadExchangeAttention:
         return lib.f2k_hx_attach(self._h, bases) == _lib.F2K_OK
 
     # ---- per step, all on one stream ------------------------------------------------------
-    @staticmethod
-    def _stream(stream):
-        import torch
-        return C.c_void_p((stream or torch.cuda.current_stream()).cuda_stream)
-
     def exchange_in(self, q_raw, k_raw, v, gamma_q, gamma_k, cos_local, sin_local, eps: float, stream=None) -> bool:
         """q_raw, k_raw, v: [1, seq_local, n_heads, 128] bf16; cos_local/sin_local: this rank's rows
         of the RoPE tables. Normalises + rotates Q and K and sends every head to its rank."""
         p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
         return lib.f2k_hx_exchange_in(self._h, p(q_raw), p(k_raw), p(v), p(gamma_q), p(gamma_k), p(cos_local),
-                                      p(sin_local), eps, self._stream(stream)) == _lib.F2K_OK
+                                      p(sin_local), eps, stream_handle(stream)) == _lib.F2K_OK
 
     def exchange_in_copy(self, q_raw, k_raw, v, gamma_q, gamma_k, cos_local, sin_local, eps: float, stream=None) -> bool:
         """exchange_in with the copy engines doing the transfers (one local prologue kernel, then
@@ -113,23 +109,23 @@ class HeadExchangeAttention:
         launches behind it runs while the copies are on their way."""
         p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
         return lib.f2k_hx_exchange_in_copy(self._h, p(q_raw), p(k_raw), p(v), p(gamma_q), p(gamma_k), p(cos_local),
-                                           p(sin_local), eps, self._stream(stream)) == _lib.F2K_OK
+                                           p(sin_local), eps, stream_handle(stream)) == _lib.F2K_OK
 
     def forward(self, q_raw, k_raw, v, gamma_q, gamma_k, cos_local, sin_local, eps: float, stream=None) -> bool:
         """exchange_in + attend as one kernel (the exchange runs on the attention kernel's spare
         warps and hides under the attention). One process per GPU, or world == 1."""
         p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
         return lib.f2k_hx_forward(self._h, p(q_raw), p(k_raw), p(v), p(gamma_q), p(gamma_k), p(cos_local),
-                                  p(sin_local), eps, self._stream(stream)) == _lib.F2K_OK
+                                  p(sin_local), eps, stream_handle(stream)) == _lib.F2K_OK
 
     def attend(self, stream=None) -> bool:
-        return lib.f2k_hx_attend(self._h, self._stream(stream)) == _lib.F2K_OK
+        return lib.f2k_hx_attend(self._h, stream_handle(stream)) == _lib.F2K_OK
 
     def output(self, stream=None):
         """Makes the stream wait for every rank's contribution; returns this rank's
         [1, seq_local, n_heads, 128] output (a view into the exchange buffer)."""
         o = C.c_void_p()
-        if lib.f2k_hx_output(self._h, C.byref(o), self._stream(stream)) != _lib.F2K_OK:
+        if lib.f2k_hx_output(self._h, C.byref(o), stream_handle(stream)) != _lib.F2K_OK:
             return None
         return _tensor_from_ptr(o.value, (1, self.seq_local, self.n_heads, self.head_dim))
 

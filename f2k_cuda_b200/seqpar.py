@@ -16,6 +16,7 @@ import ctypes as C
 
 from . import _lib
 from ._lib import SeqParConfig, lib
+from ._stream import stream_handle
 
 
 def shard_bounds(seq: int, world: int, rank: int) -> tuple[int, int]:
@@ -105,11 +106,8 @@ class SequenceParallelAttention:
     def forward(self, q_local, o_local, overlap: bool = True, stream=None) -> bool:
         """Attention of this rank's queries over all ranks' keys/values. `stream` is the compute
         stream this rank wrote its K/V on; the pulls run on a copy stream owned by the handle."""
-        import torch
-        if stream is None:
-            stream = torch.cuda.current_stream()
         rc = lib.f2k_seqpar_forward(self._h, C.c_void_p(q_local.data_ptr()), C.c_void_p(o_local.data_ptr()),
-                                    int(overlap), C.c_void_p(stream.cuda_stream), None)
+                                    int(overlap), stream_handle(stream), None)
         return rc == _lib.F2K_OK
 
     def device_status(self) -> int:
@@ -129,13 +127,10 @@ class SequenceParallelAttention:
 def qk_norm_rope(x, y, gamma, cos_table, sin_table, eps: float, stream=None) -> bool:
     """y = RoPE(RMSNorm(x) * gamma) per head row of x [batch, seq, heads, 128]; position = token
     index, so a sequence shard passes its own rows of the tables."""
-    import torch
-    if stream is None:
-        stream = torch.cuda.current_stream()
     b, s, h, _ = x.shape
     p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
     return lib.f2k_qk_norm_rope_bf16(p(x), p(y), p(gamma), p(cos_table), p(sin_table), b, s, h, eps,
-                                     C.c_void_p(stream.cuda_stream)) == _lib.F2K_OK
+                                     stream_handle(stream)) == _lib.F2K_OK
 
 
 def _tensor_from_ptr(ptr: int, shape):
