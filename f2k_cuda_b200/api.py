@@ -115,6 +115,7 @@ class _Module:
         the GPU. Asynchronous on the stream."""
         if not self.ok():
             return False
+        _check_bf16(hQ_txt, hK_txt, hV_txt, hQ_img, hK_img, hV_img, hO_txt, hO_img, *gammas)
         return lib.f2k_attn_forward_fused_host(
             self._h, _p(hQ_txt), _p(hK_txt), _p(hV_txt), _p(hQ_img), _p(hK_img), _p(hV_img),
             *[_p(g) for g in gammas], *[_p(t) for t in tables], eps, _p(hO_txt), _p(hO_img),
