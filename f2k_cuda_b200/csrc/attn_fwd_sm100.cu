@@ -778,9 +778,8 @@ static size_t attn_fwd_smem_bytes_exchange() { return kSmemUsed + 1024; }       
 // handle is created, so that the first launch does not have to load code: loading may
 // synchronise the device, which must not happen while a stream is parked on a wait that only a
 // later call (or another process) can satisfy.
-cudaError_t attn_fwd_prepare() {
+static cudaError_t prepare_on(int& dev) {       // dev: receives the current device
     static bool configured[64] = {};
-    int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 64 && configured[dev]) return cudaSuccess;
@@ -799,8 +798,14 @@ cudaError_t attn_fwd_prepare() {
     return cudaSuccess;
 }
 
+cudaError_t attn_fwd_prepare() {
+    int dev = 0;
+    return prepare_on(dev);
+}
+
 cudaError_t attn_fwd_launch(const AttnParams& params, cudaStream_t stream) {
-    cudaError_t e = attn_fwd_prepare();
+    int dev = 0;
+    cudaError_t e = prepare_on(dev);
     if (e != cudaSuccess) return e;
     AttnParams p = params;
     if (p.wait_limit_clk <= 0) p.wait_limit_clk = kDefaultWaitClk;
@@ -814,9 +819,8 @@ cudaError_t attn_fwd_launch(const AttnParams& params, cudaStream_t stream) {
     p.waits_for_words = peer_words ? 1 : 0;
     dim3 grid(p.n_heads, (p.n_q_tiles + 1) / 2, p.batch);
     if (!p.grid_head_fastest) {
-        int dev = 0, sms = 0;
-        e = cudaGetDevice(&dev);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        int sms = 0;
+        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return e;
         p.plan = cta_plan(p.n_q_tiles, p.n_heads * p.batch, sms);
         grid = dim3(p.plan.n_ctas);
